@@ -295,7 +295,7 @@ int itp2d_hermitian_eigensolve(int n, const double* A, double* evals, double* ev
  * applications whose memory manager owns the whole device, or loops that
  * cannot afford the synchronisation of cudaMalloc/cudaFree. It allocates
  * nothing; its temporaries live in one fixed device array of this library
- * (about 1.6 MB, resident on every GPU that loads the library until exit).
+ * (about 2 MB, resident on every GPU that loads the library until exit).
  * n above ITP2D_NOALLOC_MAX_N returns ITP2D_E_INVALID. All calls share that
  * array, so calls that overlap on the GPU race: serialise them. Every call
  * looks up the array's address on the current device (a device reset leaves

@@ -1,16 +1,16 @@
-// Block Jacobi eigensolver for the overlap matrix at large k.
+// Block Jacobi eigensolver of the overlap matrix.
 //
-// Same decomposition as the scalar kernel in jacobi.cu (and the same output
-// conventions), organised for fewer grid-wide rounds: the padded index range
-// is cut into blocks of BS, blocks are paired round-robin (k/BS - 1 rounds per
-// sweep), and each round r has two phases:
+// Cyclic two-sided Jacobi (A <- J^H A J, V <- V J) organised for few grid-wide
+// rounds: the padded index range is cut into blocks of BS, blocks are paired
+// round-robin (k/BS - 1 rounds per sweep), and each round r has two phases:
 //   1. one CTA per block pair sweeps the 2BS x 2BS Hermitian subproblem in
 //      shared memory with cyclic Jacobi (CTA barriers only), leaving its
 //      2BS x 2BS unitary Q_r in global memory and the rotated subproblem as
 //      the diagonal pair block of A_r;
 //   2. every other 2BS x 2BS block of A_r becomes Q_r^H A_{r-1} Q_r (row and
-//      column pairs) and every slab of 2BS rows of V becomes V Q_r, both as
-//      FP64 DMMA products staged in shared memory.
+//      column pairs; the blocks above the diagonal, mirrored) and every slab
+//      of 2BS rows of V becomes V Q_r, both as FP64 DMMA products staged in
+//      shared memory.
 // The phases are pipelined: one grid barrier separates supersteps, and
 // superstep t runs phase 1 of round t on one set of CTAs while the others run
 // phase 2 of round t - 1. Phase 1 of round t therefore builds its subproblem
@@ -45,13 +45,12 @@ namespace {
 constexpr int BS = 16;        // block size
 constexpr int MS = 32;        // subproblem size: two blocks
 constexpr int NR = MS / 2;    // rotations per inner round
-constexpr int LD = MS + 4;    // padded row length (doubles): conflict-free DMMA fragments
-constexpr int PL = MS * LD;   // doubles per plane
-// 512 threads, one CTA per SM: in an inner round, threads [0, 256) update the
-// 256 2 x 2 blocks of M while threads [256, 512) rotate the columns of Q; the
-// two halves of a phase-2 CTA work on separate products.
+constexpr int LD = MS + 4;    // padded row length (complex): conflict-free 16-byte DMMA fragments
+constexpr int OP = MS * LD;   // elements of one product operand
+constexpr int LDM = MS + 1;   // row length of M: conflict-free rows and columns
+// 512 threads, one CTA per SM: an inner sweep gives its warps separate roles
+// (inner_sweep); the two halves of a phase-2 CTA work on separate products.
 constexpr int kThreads = 512;
-constexpr int kMThreads = NR * NR;
 constexpr double kTauFinal = 3e-9;
 // Rounds between full inner sweeps (within-block pairs rotated again); every
 // 16th round measured best on k = 500 (fewer outer sweeps for little cost).
@@ -73,17 +72,19 @@ __device__ __forceinline__ int rr_player(int pos, int r, int npos) {
 __device__ __forceinline__ int gidx(int i, int P, int Q) { return i < BS ? P * BS + i : Q * BS + (i - BS); }
 
 struct Shared {
-	// phase 1: [0,1] M, [2,3] Q, [4,5] formation operands; phase 2: half h of
-	// the CTA uses [6h, 6h + 6): X/T, Q_r, Q_c
-	double pl[12][PL];
+	// phase 1: op[0] and op[1], op[2] formation operands, then the two buffers of
+	// the subproblem M (row length LDM); phase 2: half h of the CTA uses op[6h,
+	// 6h + 6), two stages of (X, Q_c, Q_r), the next item's copied in while the
+	// current one is multiplied
+	double2 op[12][OP];
 	// rotations of two consecutive inner rounds (round r in buffer r & 1)
-	double2 rst[2][NR];                          // (sin, tau)
+	double2 rst[2][NR];                          // (sin, tau), (0, 0): none
 	double2 re[2][NR];                           // e = c / |c|
-	double rap[2][NR], raq[2][NR];               // M(p, p), M(q, q) after the round
-	int rpq[2][NR];                              // p | q << 8 | applied << 16
 	int next[2];  // phase-2 item of each CTA half
 	int cnt;                                     // counted rotations of the current outer sweep
 	unsigned long long tmax;                     // largest tangent (bits of a non-negative double)
+	// Subproblem buffer b, only the upper triangle (row <= column) in use.
+	__device__ double2* m(int b) { return op[3] + b * OP; }
 };
 
 // Reciprocal and reciprocal square root in double precision by Newton-Raphson
@@ -109,40 +110,17 @@ __device__ __forceinline__ double rsqrt_nr(double x) {
 __device__ __forceinline__ int exp2i(double x) { return (int)((__double_as_longlong(x) >> 52) & 0x7ff) - 1023; }
 __device__ __forceinline__ double pow2i(int e) { return __longlong_as_double((long long)(e + 1023) << 52); }
 
-// Rotation of the local pair (p, q) of the subproblem in planes (mr, mi).
-// With d = (b - a) / 2, r = sqrt(d^2 + |c|^2), u = |d| + r and w = 2 r u, the
-// rotation of the smaller angle has tan = |c| / u, cos = u / sqrt(w) and
-// |sin| = |c| / sqrt(w) (cos^2 + sin^2 = (u^2 + |c|^2) / w = 1), and
-// tau = sin / (1 + cos) = |c| / (sqrt(w) + u): three dependent Newton-refined
-// reciprocal (square root) steps. d and c are scaled by the power of two of
-// max(|d|, |c|), and c alone by its own for e = c / |c|, so that every refined
-// estimate starts inside float range; exponents beyond +-1000 take the same
-// formulas through scalbn.
-// The pair has M(p, p) = a, M(q, q) = b, M(p, q) = (cr, ci); the rotation
-// goes to rotation buffer buf, slot j. Counted rotations and the largest
-// counted tangent accumulate in the caller's registers (cnt, tmax) and are
-// reduced once per inner sweep.
-__device__ __forceinline__ void inner_rotation(Shared& sh, int buf, int j, int p, int q, double a, double b,
-		double cr, double ci, double tol, int& cnt, double& tmax) {
-	const double c2 = cr * cr + ci * ci;
-	const double scale2 = fabs(a) * fabs(b);
-	sh.rap[buf][j] = a;
-	sh.raq[buf][j] = b;
-	sh.rpq[buf][j] = p | q << 8;
-	if (!(c2 > 0.0 && c2 > tol * tol * scale2)) return;
-	const double d = 0.5 * (b - a);
+// sin, tau = tan(angle / 2), e and tan of a rotation in double precision
+// throughout, for pairs whose exponents leave the range of the single-precision
+// set-up below: with u = |d| + r and w = 2 r u, cos = u / sqrt(w), |sin| =
+// |c| / sqrt(w) and |tau| = |c| / (sqrt(w) + u), d and c scaled by exact powers
+// of two.
+__device__ __noinline__ void rotation_wide(double d, double cr, double ci, double& s, double& tau, double& er,
+		double& ei, double& t) {
 	const double ad = fabs(d);
 	const double mc = fmax(fabs(cr), fabs(ci));
-	const double m = fmax(ad, mc);
-	int ex = exp2i(m), exc = exp2i(mc);
-	const bool fast = ex > -1000 && ex < 1000 && exc > -1000 && exc < 1000;
-	if (!fast) {
-		ex = ilogb(m);
-		exc = ilogb(mc);
-	}
-	const double sc = fast ? pow2i(-ex) : scalbn(1.0, -ex);
-	const double scc = fast ? pow2i(-exc) : scalbn(1.0, -exc);
-	// ratios in units of 2^ex: max(dn, |crn|, |cin|) in [1, 2)
+	const int ex = ilogb(fmax(ad, mc)), exc = ilogb(mc);
+	const double sc = scalbn(1.0, -ex), scc = scalbn(1.0, -exc);
 	const double dn = ad * sc, crn = cr * sc, cin = ci * sc;
 	const double cn2 = crn * crn + cin * cin;
 	const double rn2 = dn * dn + cn2;         // [1, 12)
@@ -151,32 +129,124 @@ __device__ __forceinline__ void inner_rotation(Shared& sh, int buf, int j, int p
 	const double wn = 2.0 * rn * un;          // [2, 38)
 	const double qn = rsqrt_nr(wn);
 	const double cn = sqrt(cn2);
-	const double t = cn * rcp_nr(un);
-	if (t == 0.0) return;
-	// e = c / |c| from c scaled by its own exponent: crs^2 + cis^2 in [1, 8)
+	t = cn * rcp_nr(un);
 	const double crs = cr * scc, cis = ci * scc;
 	const double ec = rsqrt_nr(crs * crs + cis * cis);
 	const double sg = d < 0 ? -1.0 : 1.0;
-	const double sw = wn * qn;                 // sqrt(w)
-	const double cabs = fast ? cn * pow2i(ex) : scalbn(cn, ex);
-	sh.rst[buf][j] = make_double2(sg * cn * qn, sg * cn * rcp_nr(sw + un));  // sw + un in [2.4, 12)
-	sh.re[buf][j] = make_double2(crs * ec, cis * ec);
-	sh.rap[buf][j] = a - sg * t * cabs;
-	sh.raq[buf][j] = b + sg * t * cabs;
-	sh.rpq[buf][j] = p | q << 8 | 1 << 16;
-	if (c2 > kNoiseRel * kNoiseRel * scale2) {
+	s = sg * cn * qn;
+	tau = sg * cn * rcp_nr(wn * qn + un);
+	er = crs * ec;
+	ei = cis * ec;
+}
+
+__device__ __forceinline__ float rsqrt_approx(float x) {
+	float y;
+	asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+	return y;
+}
+__device__ __forceinline__ float rcp_approx(float x) {
+	float y;
+	asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+	return y;
+}
+
+// A rotation J = [[cos, s e], [-s conj(e), cos]], cos = 1 - s tau; s = tau = 0
+// and e = 1 when the pair is not rotated.
+struct Rotation {
+	double s, tau, er, ei;
+};
+
+// Rotation that (nearly) zeroes c = A_pq of the pair with diagonals a, b. A
+// Jacobi rotation has to be unitary to double precision, but its angle need
+// not be exact: the angle comes from single precision (relative error about
+// 1e-7, which leaves 1e-7 |c| in place of the zero, computed by rotated_pair),
+// and the unitary is then built from it in double precision:
+//   tau = tan(angle / 2) = u (the single-precision value, exactly),
+//   sin = 2 u / (1 + u^2), cos = 1 - sin tau = (1 - u^2) / (1 + u^2),
+//   e   = c / |c| with |e| corrected to one by the series of (1 - x)^{-1/2}.
+// This replaces a chain of five Newton-refined double-precision square roots
+// and reciprocals (about 40 dependent operations of 8.5 cycles) by about
+// eight, on the critical path of every inner round. Counted rotations and the
+// largest counted tangent accumulate in cnt and tmax.
+__device__ __forceinline__ Rotation make_rotation(double a, double b, double cr, double ci, double tol, int& cnt,
+		double& tmax) {
+	const double c2 = cr * cr + ci * ci;
+	const double scale2 = fabs(a) * fabs(b);
+	const double d = 0.5 * (b - a);
+	const double mc = fmax(fabs(cr), fabs(ci));
+	const bool want = c2 > 0.0 && c2 > tol * tol * scale2;
+	// squares and quotients of d and c stay inside the single-precision range
+	const bool narrow = mc > 1e-18 && mc < 1e18 && fabs(d) < 1e18;
+	const float x = (float)cr, y = (float)ci;
+	const float dn = fabsf((float)d);
+	const float h2 = x * x + y * y;
+	const float ih = rsqrt_approx(h2);
+	const float q2 = fmaf(dn, dn, h2);
+	const float v = h2 * ih * rcp_approx(fmaf(q2, rsqrt_approx(q2), dn));  // tan = |c| / (|d| + r) in [0, 1]
+	const float w = v * v, w2 = w * w, w4 = w2 * w2;
+	// tan(angle / 2) = v / (1 + sqrt(1 + w)) and 1 / (1 + u^2) = (1 + 1 / sqrt(1 + w)) / 2
+	// from Chebyshev fits on [0, 1] (relative errors 6e-8 and 1.8e-7)
+	const float u = v * fmaf(w4, fmaf(w2, fmaf(w, -0.00104739867f, 0.00552987031f), fmaf(w, -0.0140554882f, 0.0248493936f)),
+			fmaf(w2, fmaf(w, -0.0385012144f, 0.0624355158f), fmaf(w, -0.124997111f, 0.499999978f)));
+	const double q0 = (double)fmaf(w4,
+			fmaf(w2, fmaf(w, -0.00630942694f, 0.0319823643f), fmaf(w, -0.0757951591f, 0.118910862f)),
+			fmaf(w2, fmaf(w, -0.152307005f, 0.18705187f), fmaf(w, -0.249980073f, 0.999999852f)));
+	double t = (double)v;
+	const double ud = (double)u;
+	const double r1 = fma(-fma(ud, ud, 1.0), q0, 1.0);
+	const double inv = fma(q0, fma(r1, r1, r1), q0);  // 1 / (1 + u^2) to r1^3, about 1e-20
+	const double e0 = (double)(x * ih), e1 = (double)(y * ih);
+	const double dl = fma(-e1, e1, fma(-e0, e0, 1.0));  // 1 - |e|^2, about 1e-7
+	const double f = fma(dl, fma(dl, 0.375, 0.5), 1.0);
+	Rotation R;
+	R.tau = d < 0 ? -ud : ud;
+	R.s = 2.0 * R.tau * inv;
+	R.er = e0 * f;
+	R.ei = e1 * f;
+	if (want && !narrow) rotation_wide(d, cr, ci, R.s, R.tau, R.er, R.ei, t);
+	if (!want || t == 0.0) {
+		R.s = R.tau = R.ei = 0.0;
+		R.er = 1.0;
+	} else if (c2 > kNoiseRel * kNoiseRel * scale2) {
 		cnt++;
 		tmax = fmax(tmax, t);
 	}
+	return R;
 }
 
-// Rotation j of an inner round from the subproblem in shared memory.
-__device__ __forceinline__ void inner_rotation_sm(Shared& sh, int buf, int j, int p, int q, double tol, int& cnt,
-		double& tmax) {
-	const double* mr = sh.pl[0];
-	const double* mi = sh.pl[1];
-	inner_rotation(sh, buf, j, p, q, mr[p * LD + p], mr[q * LD + q], mr[p * LD + q], mi[p * LD + q], tol, cnt,
-			tmax);
+// J^H [[a, c], [conj(c), b]] J: with w = conj(e) c and d = (b - a) / 2 the
+// diagonals are a + h and b - h, h = 2 s (s d - cos Re w), and the off-diagonal
+// e (Re w - 2 s (s Re w + cos d) + i Im w), which vanishes for the exact angle.
+__device__ __forceinline__ void rotated_pair(const Rotation& R, double& a, double& b, double& cr, double& ci) {
+	const double cs = fma(-R.s, R.tau, 1.0);
+	const double d = 0.5 * (b - a);
+	const double wr = R.er * cr + R.ei * ci;
+	const double wi = R.er * ci - R.ei * cr;
+	const double h = 2.0 * R.s * (R.s * d - cs * wr);
+	const double g = wr - 2.0 * R.s * (R.s * wr + cs * d);
+	a += h;
+	b -= h;
+	cr = R.er * g - R.ei * wi;
+	ci = R.er * wi + R.ei * g;
+}
+
+// Element (x, y) of the Hermitian M kept as its upper triangle.
+__device__ __forceinline__ int m_at(int x, int y) { return min(x, y) * LDM + max(x, y); }
+__device__ __forceinline__ double2 ld_m(const double2* m, int x, int y) {
+	double2 v = m[m_at(x, y)];
+	if (x > y) v.y = -v.y;
+	return v;
+}
+__device__ __forceinline__ void st_m(double2* m, int x, int y, double2 v) {
+	if (x > y) v.y = -v.y;
+	m[m_at(x, y)] = v;
+}
+
+// The index of pair position pos in round r of the circle method on MS indices.
+__device__ __forceinline__ int circle(int pos, int r) {
+	int v = pos - 1 + r;
+	if (v >= MS - 1) v -= MS - 1;
+	return pos == 0 ? 0 : v + 1;
 }
 
 // Rows p, q of J^H X with J = [[c, s e], [-s conj(e), c]] (correction form,
@@ -204,128 +274,258 @@ __device__ __forceinline__ void cols2(double s, double tau, double er, double ei
 	xsr = ysr; xsi = ysi; xtr = ytr; xti = yti;
 }
 
-// One inner sweep on the MS x MS subproblem in planes 0/1, accumulating Q in
-// planes 2/3: full (MS - 1 rounds of NR rotations over all pairs) or cross
-// (BS rounds: round r pairs p with BS + (p + r) % BS). Each round updates
-// every 2 x 2 block {p,q} x {s,t} in place as J_pq^H X J_st (threads
-// [0, 256)) while threads [256, 512) rotate the columns of Q, so the
-// subproblem crosses shared memory once per round.
-// In a cross sweep, round r + 1 pairs p with q' = BS + (p + r + 1) % BS, the
-// second index of pair p + 1 in round r; so the thread updating the block
-// (pair p, pair p + 1) of round r holds M(p, q') and finds M(p, p) and
-// M(q', q') among round r's results, and sets up rotation p of round r + 1
-// right away: one barrier per inner round.
-__device__ void inner_sweep(Shared& sh, double tol, bool full) {
-	double* mr = sh.pl[0];
-	double* mi = sh.pl[1];
-	double* qr = sh.pl[2];
-	double* qi = sh.pl[3];
-	const int tid = threadIdx.x;
-	const int rounds = full ? MS - 1 : BS;
-	int cnt = 0;
-	double tmax = 0.0;
-	if (tid < NR) {
-		const int p = full ? rr_player(tid, 0, MS) : tid;
-		const int q = full ? rr_player(MS - 1 - tid, 0, MS) : BS + tid;
-		inner_rotation_sm(sh, 0, tid, p, q, tol, cnt, tmax);
-	}
-	__syncthreads();
-	for (int r = 0; r < rounds; r++) {
-		const int cur = r & 1;
-		if (full && r > 0) {
-			if (tid < NR)
-				inner_rotation_sm(sh, cur, tid, rr_player(tid, r, MS), rr_player(MS - 1 - tid, r, MS), tol, cnt, tmax);
+// One inner sweep on the MS x MS subproblem in M buffer 0: FULL, MS - 1 rounds
+// of NR rotations over all pairs (circle method: pair j is (position j,
+// position MS - 1 - j)), or cross, BS rounds (round r pairs j with BS + (j + r)
+// % BS). The result is left in M buffer R & 1 (R rounds) and the unitary Q in
+// Qg, transposed (Qg[l * MS + i] = Q(i, l)). Three groups of warps work side by side on round r, one barrier per
+// round:
+//  * warp 0 (lane j: pair j) computes rotation r + 1 from M_r and rotation r.
+//    The two indices of pair j of round r + 1 sit in two different pairs A, B
+//    of round r, so its off-diagonal element is one element of the 2 x 2 block
+//    (A, B) rotated by rotation r; its diagonals are lane A's and lane B's,
+//    carried in registers. It also writes the rotated pairs' own 2 x 2 blocks.
+//  * warps 1, 2, 3 and 5 (one 2 x 2 block of pairs ja < jb per thread, 120 of
+//    128) form J^H M J in the other M buffer: the upper triangle only.
+//  * warps 6, 7, 9-11 and 13-15 hold Q in registers (lane j: the columns of
+//    pair j, four rows per warp) and pass the columns on through shared memory
+//    (shuffles of 64-bit values cost four times as much there: 3.7 cycles per
+//    32-bit shuffle).
+// Warps 4, 8 and 12 stay idle: warp 0 has its scheduler to itself, because its
+// chain of rotations bounds the round. Before, every warp updating M set up two rotations itself,
+// in double precision, and all of M and Q crossed shared memory: 2390 cycles
+// per cross round against 940 now (1230 per full round).
+template <bool FULL>
+__device__ __forceinline__ void inner_sweep(Shared& sh, double tol, double2* Qg) {
+	constexpr int R = FULL ? MS - 1 : BS;
+	const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+	// position of pair index j's second member in round r
+	auto second = [](int j, int r) { return FULL ? circle(MS - 1 - j, r) : BS + ((j + r) & (BS - 1)); };
+	auto first = [](int j, int r) { return FULL ? circle(j, r) : j; };
+	if (warp == 0) {
+		const int j = lane & (NR - 1);
+		int cnt = 0;
+		double tmax = 0.0;
+		int p = first(j, 0), q = second(j, 0);
+		double a = sh.m(0)[m_at(p, p)].x, b = sh.m(0)[m_at(q, q)].x;
+		double2 c = ld_m(sh.m(0), p, q);
+		Rotation ro = make_rotation(a, b, c.x, c.y, tol, cnt, tmax);
+		if (lane < NR) {
+			sh.rst[0][j] = make_double2(ro.s, ro.tau);
+			sh.re[0][j] = make_double2(ro.er, ro.ei);
+		}
+		// round r + 1's pair j: index 1 of pair A (its first or second member) and
+		// of pair B; the other members ride along in the 2 x 2 block
+		const int A = FULL ? (j == 0 ? 0 : min(j + 1, NR - 1)) : j;
+		const int B = FULL ? (j == 0 ? 1 : j - 1) : ((j + 1) & (NR - 1));
+		const bool a_first = !FULL || j < NR - 1, b_first = FULL && j == 0;
+		const double sa = a_first ? 1.0 : -1.0, sb = b_first ? 1.0 : -1.0;
+		// the block's element offsets and signs of the imaginary parts, formed
+		// one round ahead: x and y the indices that meet, xo and yo their partners
+		int x, y, o11, o21, o12, o22;
+		unsigned conj;
+		auto block = [&](int r) {
+			const int fa = first(A, r), qa = second(A, r), fb = first(B, r), qb = second(B, r);
+			x = a_first ? fa : qa;
+			y = b_first ? fb : qb;
+			const int xo = a_first ? qa : fa, yo = b_first ? qb : fb;
+			o11 = m_at(x, y);
+			o21 = m_at(xo, y);
+			o12 = m_at(x, yo);
+			o22 = m_at(xo, yo);
+			conj = (x > y ? 1u : 0u) | (xo > y ? 2u : 0u) | (x > yo ? 4u : 0u) | (xo > yo ? 8u : 0u);
+		};
+		block(0);
+		__syncthreads();
+#pragma unroll 1
+		for (int r = 0; r < R; r++) {
+			const int cur = r & 1;
+			const double2* m = sh.m(cur);
+			double2* mn = sh.m(cur ^ 1);
+			double2 m11 = m[o11], m21 = m[o21], m12 = m[o12], m22 = m[o22];
+			const double2 ta = sh.rst[cur][A], ea = sh.re[cur][A], tb = sh.rst[cur][B], eb = sh.re[cur][B];
+			// rotation r's own pair, before the loads are used
+			const int po = p, qo = q;
+			rotated_pair(ro, a, b, c.x, c.y);
+			const double ao = a, bo = b;
+			if (lane < NR) {
+				mn[m_at(po, po)] = make_double2(ao, 0.0);
+				mn[m_at(qo, qo)] = make_double2(bo, 0.0);
+				st_m(mn, po, qo, c);
+			}
+			p = x;
+			q = y;
+			if (r + 1 < R) {
+				if (conj & 1) m11.y = -m11.y;
+				if (conj & 2) m21.y = -m21.y;
+				if (conj & 4) m12.y = -m12.y;
+				if (conj & 8) m22.y = -m22.y;
+				// row x of J_A^H M: x - s (e xo + tau x), with s, tau and Im e negated
+				// for the second member
+				const double s1 = sa * ta.x, t1 = sa * ta.y, e1i = sa * ea.y;
+				const double u1r = m11.x - s1 * (ea.x * m21.x - e1i * m21.y + t1 * m11.x);
+				const double u1i = m11.y - s1 * (ea.x * m21.y + e1i * m21.x + t1 * m11.y);
+				const double u2r = m12.x - s1 * (ea.x * m22.x - e1i * m22.y + t1 * m12.x);
+				const double u2i = m12.y - s1 * (ea.x * m22.y + e1i * m22.x + t1 * m12.y);
+				// column y of the result times J_B: y - s (conj(e) yo + tau y)
+				const double s2 = sb * tb.x, t2 = sb * tb.y, e2i = sb * eb.y;
+				c.x = u1r - s2 * (eb.x * u2r + e2i * u2i + t2 * u1r);
+				c.y = u1i - s2 * (eb.x * u2i - e2i * u2r + t2 * u1i);
+				if (FULL) {
+					const double an = __shfl_sync(0xffffffffu, ao, (j + 1) & (NR - 1), NR);
+					const double bp = __shfl_sync(0xffffffffu, bo, (j - 1) & (NR - 1), NR);
+					a = j == 0 ? ao : (j == NR - 1 ? bo : an);
+					b = j == 0 ? an : bp;
+				} else {
+					b = __shfl_sync(0xffffffffu, bo, (j + 1) & (NR - 1), NR);
+				}
+				block(r + 1);
+				ro = make_rotation(a, b, c.x, c.y, tol, cnt, tmax);
+				if (lane < NR) {
+					sh.rst[cur ^ 1][j] = make_double2(ro.s, ro.tau);
+					sh.re[cur ^ 1][j] = make_double2(ro.er, ro.ei);
+				}
+			}
 			__syncthreads();
 		}
-		if (tid < kMThreads) {
-			const int ja = tid / NR, jb = tid % NR;
-			const int pa = sh.rpq[cur][ja], pb = sh.rpq[cur][jb];
-			const bool ra = pa >> 16, rb = pb >> 16;
-			const bool nx = !full && r + 1 < rounds && jb == ((ja + 1) & (NR - 1));
-			const int p = pa & 255, q = (pa >> 8) & 255, s2 = pb & 255, t2 = (pb >> 8) & 255;
-			if (ja == jb) {
-				if (ra) {
-					mr[p * LD + p] = sh.rap[cur][ja]; mi[p * LD + p] = 0.0;
-					mr[q * LD + q] = sh.raq[cur][ja]; mi[q * LD + q] = 0.0;
-					mr[p * LD + q] = 0.0; mi[p * LD + q] = 0.0;
-					mr[q * LD + p] = 0.0; mi[q * LD + p] = 0.0;
-				}
-			} else if (ra || rb || nx) {
-				double psr = mr[p * LD + s2], psi = mi[p * LD + s2], ptr = mr[p * LD + t2], pti = mi[p * LD + t2];
-				double qsr = mr[q * LD + s2], qsi = mi[q * LD + s2], qtr = mr[q * LD + t2], qti = mi[q * LD + t2];
-				if (ra) {
-					const double2 st = sh.rst[cur][ja], e = sh.re[cur][ja];
-					rows2(st.x, st.y, e.x, e.y, psr, psi, qsr, qsi);
-					rows2(st.x, st.y, e.x, e.y, ptr, pti, qtr, qti);
-				}
-				if (rb) {
-					const double2 st = sh.rst[cur][jb], e = sh.re[cur][jb];
-					cols2(st.x, st.y, e.x, e.y, psr, psi, ptr, pti);
-					cols2(st.x, st.y, e.x, e.y, qsr, qsi, qtr, qti);
-				}
-				if (ra || rb) {
-					mr[p * LD + s2] = psr; mi[p * LD + s2] = psi; mr[p * LD + t2] = ptr; mi[p * LD + t2] = pti;
-					mr[q * LD + s2] = qsr; mi[q * LD + s2] = qsi; mr[q * LD + t2] = qtr; mi[q * LD + t2] = qti;
-				}
-				if (nx)
-					inner_rotation(sh, cur ^ 1, ja, p, t2, sh.rap[cur][ja], sh.raq[cur][jb], ptr, pti, tol, cnt, tmax);
-			}
-		} else {
-			for (int e = tid - kMThreads; e < MS * NR; e += kThreads - kMThreads) {
-				const int i = e / NR, j = e % NR;
-				const int pj = sh.rpq[cur][j];
-				if (!(pj >> 16)) continue;
-				const int p = pj & 255, q = (pj >> 8) & 255;
-				double ysr = qr[i * LD + p], ysi = qi[i * LD + p], ytr = qr[i * LD + q], yti = qi[i * LD + q];
-				const double2 st = sh.rst[cur][j], ev = sh.re[cur][j];
-				cols2(st.x, st.y, ev.x, ev.y, ysr, ysi, ytr, yti);
-				qr[i * LD + p] = ysr; qi[i * LD + p] = ysi; qr[i * LD + q] = ytr; qi[i * LD + q] = yti;
-			}
+		if (lane >= NR) {
+			cnt = 0;
+			tmax = 0.0;
 		}
+		for (int o = 8; o > 0; o >>= 1) {
+			cnt += __shfl_xor_sync(0xffffffffu, cnt, o);
+			tmax = fmax(tmax, __shfl_xor_sync(0xffffffffu, tmax, o));
+		}
+		if (lane == 0 && cnt) {
+			sh.cnt += cnt;
+			const unsigned long long tb = (unsigned long long)__double_as_longlong(tmax);
+			if (tb > sh.tmax) sh.tmax = tb;
+		}
+	} else if (warp < 4 || warp == 5) {
+		// item (ja, jb), ja < jb, of the NR (NR - 1) / 2
+		const int item = (warp < 4 ? warp - 1 : 3) * 32 + lane;
+		int ja = 0, jb = 1;
+		{
+			int left = item;
+			while (ja < NR - 1 && left >= NR - 1 - ja) {
+				left -= NR - 1 - ja;
+				ja++;
+			}
+			jb = ja + 1 + left;
+		}
+		const bool on = item < NR * (NR - 1) / 2;
 		__syncthreads();
+#pragma unroll 1
+		for (int r = 0; r < R; r++) {
+			const int cur = r & 1;
+			if (on) {
+				const double2* m = sh.m(cur);
+				double2* mn = sh.m(cur ^ 1);
+				const int p = first(ja, r), q = second(ja, r), s = first(jb, r), t = second(jb, r);
+				double2 ps = ld_m(m, p, s), pt = ld_m(m, p, t), qs = ld_m(m, q, s), qt = ld_m(m, q, t);
+				const double2 ta = sh.rst[cur][ja], ea = sh.re[cur][ja], tb = sh.rst[cur][jb], eb = sh.re[cur][jb];
+				rows2(ta.x, ta.y, ea.x, ea.y, ps.x, ps.y, qs.x, qs.y);
+				rows2(ta.x, ta.y, ea.x, ea.y, pt.x, pt.y, qt.x, qt.y);
+				cols2(tb.x, tb.y, eb.x, eb.y, ps.x, ps.y, pt.x, pt.y);
+				cols2(tb.x, tb.y, eb.x, eb.y, qs.x, qs.y, qt.x, qt.y);
+				st_m(mn, p, s, ps);
+				st_m(mn, p, t, pt);
+				st_m(mn, q, s, qs);
+				st_m(mn, q, t, qt);
+			}
+			__syncthreads();
+		}
+	} else if ((warp & 3) != 0) {
+		// rows i0, i0 + 1 of Q, columns of pair j
+		const int w = warp < 8 ? warp - 6 : (warp < 12 ? warp - 7 : warp - 8);
+		const int j = lane & (NR - 1);
+		const int i0 = 4 * w + 2 * (lane >> 4);
+		const int p0 = first(j, 0), q0 = second(j, 0);
+		double2 xp[2], xq[2];
+#pragma unroll
+		for (int h = 0; h < 2; h++) {
+			xp[h] = make_double2(i0 + h == p0 ? 1.0 : 0.0, 0.0);
+			xq[h] = make_double2(i0 + h == q0 ? 1.0 : 0.0, 0.0);
+		}
+		// this warp's exchange area: [member][row h][half of the warp][column]
+		double2* xch = sh.op[5] + w * 4 * 2 * NR;
+		const int at = (lane >> 4) * NR, own = at + j, up = at + ((j + 1) & (NR - 1)), down = at + ((j - 1) & (NR - 1));
+		__syncthreads();
+#pragma unroll 1
+		for (int r = 0; r < R; r++) {
+			const double2 st = sh.rst[r & 1][j], e = sh.re[r & 1][j];
+#pragma unroll
+			for (int h = 0; h < 2; h++) cols2(st.x, st.y, e.x, e.y, xp[h].x, xp[h].y, xq[h].x, xq[h].y);
+			// the columns move on to the lanes of round r + 1's pairs
+#pragma unroll
+			for (int h = 0; h < 2; h++) {
+				xch[32 * h + own] = xq[h];
+				if (FULL) xch[64 + 32 * h + own] = xp[h];
+			}
+			__syncwarp();
+#pragma unroll
+			for (int h = 0; h < 2; h++) {
+				if (FULL) {
+					// positions move up by one around the circle, position 0 stays
+					const double2 pn = xch[64 + 32 * h + up];
+					const double2 qn = xch[32 * h + down];
+					if (j == NR - 1) xp[h] = xq[h];
+					else if (j > 0) xp[h] = pn;
+					xq[h] = j == 0 ? pn : qn;
+				} else {
+					xq[h] = xch[32 * h + up];
+				}
+			}
+			__syncthreads();  // also: the exchange area is free again
+		}
+		// after all rounds the columns are back at their places
+#pragma unroll
+		for (int h = 0; h < 2; h++) {
+			Qg[p0 * MS + i0 + h] = xp[h];
+			Qg[q0 * MS + i0 + h] = xq[h];
+		}
+	} else {
+		__syncthreads();
+#pragma unroll 1
+		for (int r = 0; r < R; r++) __syncthreads();
 	}
-	// counts and tangents of every thread that set up rotations
-	for (int o = 16; o > 0; o >>= 1) {
-		cnt += __shfl_xor_sync(0xffffffffu, cnt, o);
-		tmax = fmax(tmax, __shfl_xor_sync(0xffffffffu, tmax, o));
-	}
-	if ((tid & 31) == 0 && cnt) {
-		atomicAdd(&sh.cnt, cnt);
-		atomicMax(&sh.tmax, (unsigned long long)__double_as_longlong(tmax));
-	}
+	__syncthreads();
 }
 
-// One 8 x 8 tile of the complex product A B (32-deep operands given as plane
-// pairs) by one warp with FP64 DMMA: acc (h) of lane holds output row
-// row0 + (lane >> 2), column col0 + 2 (lane & 3) + h. A element (i, m) at
-// a_re[i * as_i + m * as_m], B element (m, l) at b_re[m * LD + l]; conjA
-// conjugates A.
-__device__ __forceinline__ void ctile(int lane, const double* ar, const double* ai, int as_i, int as_m, bool conjA,
-		const double* br, const double* bi, int row0, int col0, double (&cr)[2], double (&ci)[2]) {
-	const int i = row0 + (lane >> 2);
-	const int l = col0 + (lane >> 2);
-	cr[0] = cr[1] = ci[0] = ci[1] = 0.0;
+// NT adjacent 8 x 8 tiles of the complex product C(i, l) = sum_m A(i, m) B(m, l)
+// (32 deep) by one warp with FP64 DMMA, both operands kept with m along their
+// rows: A(i, m) at A[i * LD + m] (conjugated with CONJ), B(m, l) at
+// B[l * LD + m]. Lane: rows row0 + (lane >> 2), columns col0 + 8 b + 2 (lane & 3)
+// + h of accumulator (b, h).
+template <int NT, bool CONJ>
+__device__ __forceinline__ void ctiles(int lane, const double2* A, const double2* B, int row0, int col0,
+		double (&cr)[NT][2], double (&ci)[NT][2]) {
+	const double2* a0 = A + (row0 + (lane >> 2)) * LD + (lane & 3);
+	const double2* b0 = B + (col0 + (lane >> 2)) * LD + (lane & 3);
+#pragma unroll
+	for (int b = 0; b < NT; b++) cr[b][0] = cr[b][1] = ci[b][0] = ci[b][1] = 0.0;
 #pragma unroll
 	for (int kk = 0; kk < MS; kk += 4) {
-		const int m = kk + (lane & 3);
-		const double far = ar[i * as_i + m * as_m];
-		const double fai = conjA ? -ai[i * as_i + m * as_m] : ai[i * as_i + m * as_m];
-		const double fbr = br[m * LD + l], fbi = bi[m * LD + l];
-		dmma(cr[0], cr[1], far, fbr);
-		dmma(cr[0], cr[1], -fai, fbi);
-		dmma(ci[0], ci[1], far, fbi);
-		dmma(ci[0], ci[1], fai, fbr);
+		double2 a = a0[kk];
+		if (CONJ) a.y = -a.y;
+#pragma unroll
+		for (int b = 0; b < NT; b++) {
+			const double2 v = b0[b * 8 * LD + kk];
+			dmma(cr[b][0], cr[b][1], a.x, v.x);
+			dmma(ci[b][0], ci[b][1], a.x, v.y);
+			dmma(cr[b][0], cr[b][1], -a.y, v.y);
+			dmma(ci[b][0], ci[b][1], a.y, v.x);
+		}
 	}
 }
 
 // Full 32 x 32 product on one half of the CTA (local warp lw of 8): warp lw
-// owns rows (lw >> 1) * 8 .. + 8 and columns (lw & 1) * 16 .. + 16 (tiles b).
-__device__ __forceinline__ void half_gemm(int lt, const double* ar, const double* ai, int as_i, int as_m,
-		bool conjA, const double* br, const double* bi, double (&cr)[2][2], double (&ci)[2][2]) {
+// owns rows (lw >> 1) * 8 .. + 8 and columns (lw & 1) * 16 .. + 16.
+template <bool CONJ>
+__device__ __forceinline__ void half_gemm(int lt, const double2* A, const double2* B, double (&cr)[2][2],
+		double (&ci)[2][2]) {
 	const int lane = lt & 31, lw = lt >> 5;
-#pragma unroll
-	for (int b = 0; b < 2; b++)
-		ctile(lane, ar, ai, as_i, as_m, conjA, br, bi, (lw >> 1) * 8, (lw & 1) * 16 + b * 8, cr[b], ci[b]);
+	ctiles<2, CONJ>(lane, A, B, (lw >> 1) * 8, (lw & 1) * 16, cr, ci);
 }
 
 // Output coordinates of accumulator (b, h) of half_gemm for local thread lt.
@@ -348,7 +548,7 @@ __device__ __forceinline__ int rr_position(int p, int r, int npos) {
 }
 
 // Phase 1 for pair j of round t (within-sweep round rr): forms the subproblem
-// in planes 0/1 (Q in planes 2/3 = I), sweeps it, stores Q_t and the rotated
+// (upper triangle of M buffer 0), sweeps it, stores Q_t and the rotated
 // subproblem. prev: A_{t-1} (diagonal pair blocks of round t - 1), prev2:
 // A_{t-2}, Qprev: the Q buffer of round t - 1 (t >= 1). For t = 0 the
 // subproblem is read from prev = A_{-1}, the initial matrix.
@@ -357,14 +557,11 @@ __device__ void phase1_item(Shared& sh, int j, long long t, int rounds, int nb, 
 	const int tid = threadIdx.x;
 	const int rr = (int)(t % rounds);
 	const int P = rr_player(j, rr, nb), Q = rr_player(nb - 1 - j, rr, nb);
-	double* mr = sh.pl[0];
-	double* mi = sh.pl[1];
+	double2* M = sh.m(0);
 	if (t == 0) {
 		for (int e = tid; e < MS * MS; e += kThreads) {
 			const int i = e / MS, l = e % MS;
-			const double2 v = __ldcg(prev + (long long)gidx(i, P, Q) * kp + gidx(l, P, Q));
-			mr[i * LD + l] = v.x;
-			mi[i * LD + l] = v.y;
+			M[i * LDM + l] = __ldcg(prev + (long long)gidx(i, P, Q) * kp + gidx(l, P, Q));
 		}
 	} else {
 		// the round t - 1 pairs (a, b) holding P and Q, and the halves they sit in
@@ -394,48 +591,37 @@ __device__ void phase1_item(Shared& sh, int j, long long t, int rounds, int nb, 
 			const int g0 = (half ? Q : P) * BS;
 			ld[it] = __ldcg(prev + (long long)(g0 + i) * kp + g0 + l);
 		}
+		double2 *X = sh.op[0], *Ta = sh.op[1], *Tb = sh.op[2];
 #pragma unroll
 		for (int it = 0; it < NL; it++) {
-			const int e = it * kThreads + tid, i = e / MS, l = e % MS;
-			mr[i * LD + l] = la[it].x;
-			mi[i * LD + l] = la[it].y;
-			sh.pl[2][i * LD + l] = lqa[it].x;
-			sh.pl[3][i * LD + l] = lqa[it].y;
-			sh.pl[4][i * LD + l] = lqb[it].x;
-			sh.pl[5][i * LD + l] = lqb[it].y;
+			const int e = it * kThreads + tid, o = (e / MS) * LD + e % MS;
+			X[o] = la[it];
+			Ta[o] = lqa[it];
+			Tb[o] = lqb[it];
 		}
 		__syncthreads();
 		// only the (hP, hQ) quadrant of Q_a^H A_{t-2}(a, b) Q_b enters the
-		// subproblem: T = A_{t-2}(a, b) Q_b[:, hQ half] (32 x 16: eight 8 x 8
+		// subproblem: T^T = Q_b[:, hQ half]^T A_{t-2}(a, b)^T (16 x 32: eight 8 x 8
 		// tiles, warps 0-7), then C = Q_a[:, hP half]^H T (16 x 16: four tiles,
 		// warps 0-3)
 		{
 			const int lane = tid & 31, warp = tid >> 5;
-			double cr[2], ci[2];
-			if (warp < 8)
-				ctile(lane, sh.pl[0], sh.pl[1], LD, 1, false, sh.pl[4] + hQ * BS, sh.pl[5] + hQ * BS, (warp >> 1) * 8,
-						(warp & 1) * 8, cr, ci);
+			double cr[1][2], ci[1][2];
+			if (warp < 8) ctiles<1, false>(lane, Tb + hQ * BS * LD, X, (warp & 1) * 8, (warp >> 1) * 8, cr, ci);
 			__syncthreads();
 			if (warp < 8)
 #pragma unroll
 				for (int h = 0; h < 2; h++) {
-					const int row = (warp >> 1) * 8 + (lane >> 2), col = (warp & 1) * 8 + 2 * (lane & 3) + h;
-					mr[row * LD + col] = cr[h];
-					mi[row * LD + col] = ci[h];
+					const int row = (warp & 1) * 8 + (lane >> 2), col = (warp >> 1) * 8 + 2 * (lane & 3) + h;
+					X[row * LD + col] = make_double2(cr[0][h], ci[0][h]);
 				}
 			__syncthreads();
-			if (warp < 4)
-				ctile(lane, sh.pl[2] + hP * BS, sh.pl[3] + hP * BS, 1, LD, true, sh.pl[0], sh.pl[1], (warp >> 1) * 8,
-						(warp & 1) * 8, cr, ci);
-			__syncthreads();
+			if (warp < 4) ctiles<1, true>(lane, Ta + hP * BS * LD, X, (warp >> 1) * 8, (warp & 1) * 8, cr, ci);
 			if (warp < 4)
 #pragma unroll
 				for (int h = 0; h < 2; h++) {
 					const int i = (warp >> 1) * 8 + (lane >> 2), l = BS + (warp & 1) * 8 + 2 * (lane & 3) + h;
-					mr[i * LD + l] = cr[h];
-					mi[i * LD + l] = ci[h];
-					mr[l * LD + i] = cr[h];
-					mi[l * LD + i] = -ci[h];
+					M[i * LDM + l] = make_double2(cr[0][h], ci[0][h]);
 				}
 		}
 		// diagonal blocks (P, P) and (Q, Q) of A_{t-1}
@@ -443,121 +629,156 @@ __device__ void phase1_item(Shared& sh, int j, long long t, int rounds, int nb, 
 		for (int it = 0; it < ND; it++) {
 			const int e = it * kThreads + tid;
 			const int half = e / (BS * BS), i = (e / BS) % BS, l = e % BS;
-			mr[(half * BS + i) * LD + half * BS + l] = ld[it].x;
-			mi[(half * BS + i) * LD + half * BS + l] = ld[it].y;
+			M[(half * BS + i) * LDM + half * BS + l] = ld[it];
 		}
 	}
-	for (int e = tid; e < MS * MS; e += kThreads) {
-		const int i = e / MS, l = e % MS;
-		sh.pl[2][i * LD + l] = (i == l) ? 1.0 : 0.0;
-		sh.pl[3][i * LD + l] = 0.0;
-	}
 	__syncthreads();
-	inner_sweep(sh, tol, rr % kFullEvery == 0);
 	double2* Qg = Qout + (size_t)j * MS * MS;
+	const bool full = rr % kFullEvery == 0;
+	if (full) inner_sweep<true>(sh, tol, Qg);
+	else inner_sweep<false>(sh, tol, Qg);
+	const int last = full ? (MS - 1) & 1 : BS & 1;
 	for (int e = tid; e < MS * MS; e += kThreads) {
 		const int i = e / MS, l = e % MS;
-		Qg[e] = make_double2(sh.pl[2][i * LD + l], sh.pl[3][i * LD + l]);
-		out[(long long)gidx(i, P, Q) * kp + gidx(l, P, Q)] = make_double2(mr[i * LD + l], mi[i * LD + l]);
+		const double2 v = ld_m(sh.m(last), i, l);
+		out[(long long)gidx(i, P, Q) * kp + gidx(l, P, Q)] = make_double2(v.x, i == l ? 0.0 : v.y);
 	}
 	__syncthreads();
 }
 
-// Phase 2 item w of round ro: an off-diagonal pair block of A (w < nA2) or a
-// slab of V, read from src / V, written to dst / V; on one half of the CTA
-// (the two halves take alternate items, each with its own planes and named
-// barrier).
-__device__ void phase2_item(Shared& sh, int half, int w, int ro, int nb, int np, int kp, const double2* src,
-		double2* dst, double2* V, const double2* Qr) {
-	const int lt = threadIdx.x & (kThreads / 2 - 1);
-	double* xr = sh.pl[6 * half + 0];
-	double* xi = sh.pl[6 * half + 1];
-	double* ar = sh.pl[6 * half + 2];
-	double* ai = sh.pl[6 * half + 3];
-	double* br = sh.pl[6 * half + 4];
-	double* bi = sh.pl[6 * half + 5];
-	const int nA2 = np * (np - 1);
-	constexpr int NH = MS * MS / (kThreads / 2);  // elements per thread and operand
-	double cr[2][2], ci[2][2];
-	if (w < nA2) {
-		const int jr = w / (np - 1);
-		int jc = w % (np - 1);
-		if (jc >= jr) jc++;
-		const int Pr = rr_player(jr, ro, nb), Qr_ = rr_player(nb - 1 - jr, ro, nb);
-		const int Pc = rr_player(jc, ro, nb), Qc = rr_player(nb - 1 - jc, ro, nb);
-		// all global loads of the item at once, then the shared-memory stores
-		double2 lx[NH], la[NH], lb[NH];
-#pragma unroll
-		for (int it = 0; it < NH; it++) {
-			const int e = it * (kThreads / 2) + lt, i = e / MS, l = e % MS;
-			lx[it] = __ldcg(src + (long long)gidx(i, Pr, Qr_) * kp + gidx(l, Pc, Qc));
-			la[it] = __ldcg(Qr + (size_t)jr * MS * MS + e);
-			lb[it] = __ldcg(Qr + (size_t)jc * MS * MS + e);
-		}
-#pragma unroll
-		for (int it = 0; it < NH; it++) {
-			const int e = it * (kThreads / 2) + lt, o = (e / MS) * LD + e % MS;
-			xr[o] = lx[it].x;
-			xi[o] = lx[it].y;
-			ar[o] = la[it].x;
-			ai[o] = la[it].y;
-			br[o] = lb[it].x;
-			bi[o] = lb[it].y;
-		}
-		half_sync(half);
-		half_gemm(lt, xr, xi, LD, 1, false, br, bi, cr, ci);  // T = X Qc
-		half_sync(half);
-#pragma unroll
-		for (int b = 0; b < 2; b++)
-#pragma unroll
-			for (int h = 0; h < 2; h++) {
-				int row, col;
-				half_rc(lt, b, h, row, col);
-				xr[row * LD + col] = cr[b][h];
-				xi[row * LD + col] = ci[b][h];
-			}
-		half_sync(half);
-		// C = Qr^H T: A(i, m) = conj(Qr(m, i))
-		half_gemm(lt, ar, ai, 1, LD, true, xr, xi, cr, ci);
-#pragma unroll
-		for (int b = 0; b < 2; b++)
-#pragma unroll
-			for (int h = 0; h < 2; h++) {
-				int row, col;
-				half_rc(lt, b, h, row, col);
-				dst[(long long)gidx(row, Pr, Qr_) * kp + gidx(col, Pc, Qc)] = make_double2(cr[b][h], ci[b][h]);
-			}
+// Phase 2 item w of a round: an off-diagonal pair block (jr, jc) of A above the
+// diagonal (its mirror image is written with it), or the slab jr of V (32
+// rows) for the pair jc.
+struct Item {
+	int jr, jc;
+	bool is_v;
+};
+__device__ __forceinline__ Item item_of(int w, int np) {
+	const int nA2 = np * (np - 1) / 2;
+	Item it;
+	it.is_v = w >= nA2;
+	if (it.is_v) {
+		it.jr = (w - nA2) / np;
+		it.jc = (w - nA2) % np;
 	} else {
-		const int v = w - nA2;
-		const int rb = v / np, jc = v % np;
-		const int Pc = rr_player(jc, ro, nb), Qc = rr_player(nb - 1 - jc, ro, nb);
-		double2 lx[NH], lb[NH];
+		// pair w of the upper triangle jr < jc, by columns
+		int jc = (int)((1.0f + sqrtf(1.0f + 8.0f * (float)w)) * 0.5f);
+		while (jc * (jc - 1) / 2 > w) jc--;
+		while ((jc + 1) * jc / 2 <= w) jc++;
+		it.jc = jc;
+		it.jr = w - jc * (jc - 1) / 2;
+	}
+	return it;
+}
+
+__device__ __forceinline__ void cp16(double2* dst, const double2* src) {
+	asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src)
+			: "memory");
+}
+
+// Starts the copies of an item's operands into stage st (X, Q_c, Q_r) by one
+// half of the CTA; one cp.async group per call.
+__device__ __forceinline__ void phase2_fetch(double2 (*st)[OP], const Item& it, int lt, int ro, int nb, int kp,
+		const double2* src, const double2* V, const double2* Qr) {
+	const int Pc = rr_player(it.jc, ro, nb), Qc = rr_player(nb - 1 - it.jc, ro, nb);
+	const int Pr = it.is_v ? 2 * it.jr : rr_player(it.jr, ro, nb);
+	const int Qr_ = it.is_v ? 2 * it.jr + 1 : rr_player(nb - 1 - it.jr, ro, nb);
+	const double2* X = it.is_v ? V : src;
 #pragma unroll
-		for (int it = 0; it < NH; it++) {
-			const int e = it * (kThreads / 2) + lt, i = e / MS, l = e % MS;
-			lx[it] = __ldcg(V + (long long)(rb * MS + i) * kp + gidx(l, Pc, Qc));
-			lb[it] = __ldcg(Qr + (size_t)jc * MS * MS + e);
-		}
-#pragma unroll
-		for (int it = 0; it < NH; it++) {
-			const int e = it * (kThreads / 2) + lt, o = (e / MS) * LD + e % MS;
-			xr[o] = lx[it].x;
-			xi[o] = lx[it].y;
-			br[o] = lb[it].x;
-			bi[o] = lb[it].y;
-		}
-		half_sync(half);
-		half_gemm(lt, xr, xi, LD, 1, false, br, bi, cr, ci);  // V Qc
+	for (int h = 0; h < MS * MS / (kThreads / 2); h++) {
+		const int e = h * (kThreads / 2) + lt, i = e / MS, l = e % MS, o = i * LD + l;
+		cp16(st[0] + o, X + (long long)gidx(i, Pr, Qr_) * kp + gidx(l, Pc, Qc));
+		cp16(st[1] + o, Qr + (size_t)it.jc * MS * MS + e);
+		if (!it.is_v) cp16(st[2] + o, Qr + (size_t)it.jr * MS * MS + e);
+	}
+	asm volatile("cp.async.commit_group;\n" ::: "memory");
+}
+
+// The products of an item from stage st, written to dst or V.
+__device__ __forceinline__ void phase2_item(double2 (*st)[OP], const Item& it, int half, int lt, int ro, int nb,
+		int kp, double2* dst, double2* V) {
+	const int Pc = rr_player(it.jc, ro, nb), Qc = rr_player(nb - 1 - it.jc, ro, nb);
+	double cr[2][2], ci[2][2];
+	if (it.is_v) {
+		half_gemm<false>(lt, st[0], st[1], cr, ci);  // V Q_c
 #pragma unroll
 		for (int b = 0; b < 2; b++)
 #pragma unroll
 			for (int h = 0; h < 2; h++) {
 				int row, col;
 				half_rc(lt, b, h, row, col);
-				V[(long long)(rb * MS + row) * kp + gidx(col, Pc, Qc)] = make_double2(cr[b][h], ci[b][h]);
+				V[(long long)(it.jr * MS + row) * kp + gidx(col, Pc, Qc)] = make_double2(cr[b][h], ci[b][h]);
 			}
+		return;
 	}
+	const int Pr = rr_player(it.jr, ro, nb), Qr_ = rr_player(nb - 1 - it.jr, ro, nb);
+	half_gemm<false>(lt, st[1], st[0], cr, ci);  // T^T = Q_c^T X^T
 	half_sync(half);
+#pragma unroll
+	for (int b = 0; b < 2; b++)
+#pragma unroll
+		for (int h = 0; h < 2; h++) {
+			int row, col;
+			half_rc(lt, b, h, row, col);
+			st[0][row * LD + col] = make_double2(cr[b][h], ci[b][h]);
+		}
+	half_sync(half);
+	half_gemm<true>(lt, st[2], st[0], cr, ci);  // Q_r^H T
+#pragma unroll
+	for (int b = 0; b < 2; b++)
+#pragma unroll
+		for (int h = 0; h < 2; h++) {
+			int row, col;
+			half_rc(lt, b, h, row, col);
+			const long long gr = gidx(row, Pr, Qr_), gc = gidx(col, Pc, Qc);
+			dst[gr * kp + gc] = make_double2(cr[b][h], ci[b][h]);
+			dst[gc * kp + gr] = make_double2(cr[b][h], -ci[b][h]);
+		}
+}
+
+// The items of round ro that one half of the CTA takes: handed out by the
+// round's counter, the next one's operands in flight (cp.async, two stages)
+// during the products of the current one. Bound: DMMA issue and the operands'
+// L2 traffic (48 KB in, 32 KB out per block of A); whole eigensolves, upper
+// triangle and copies ahead against all blocks with loads in line: 21.4 -> 17.7
+// ms at k = 1000 (9 sweeps), 161 -> 124 ms at k = 2000 (10 sweeps).
+__device__ void phase2(Shared& sh, int ro, int nb, int np, int nW, int kp, const double2* src, double2* dst,
+		double2* V, const double2* Qr, int* ctr) {
+	const int half = threadIdx.x / (kThreads / 2), lt = threadIdx.x & (kThreads / 2 - 1);
+	auto take = [&]() {
+		if (lt == 0) sh.next[half] = atomicAdd(ctr, 1);
+		half_sync(half);
+		const int w = sh.next[half];
+		half_sync(half);
+		return w;
+	};
+	double2(*st)[OP] = sh.op + 6 * half;
+	int w = take(), cur = 0;
+	if (w >= nW) return;
+	Item it = item_of(w, np);
+	phase2_fetch(st, it, lt, ro, nb, kp, src, V, Qr);
+	int wn = take();
+	while (w < nW) {
+		Item nx{};
+		if (wn < nW) {
+			nx = item_of(wn, np);
+			phase2_fetch(st + 3 * (cur ^ 1), nx, lt, ro, nb, kp, src, V, Qr);
+			asm volatile("cp.async.wait_group 1;\n" ::: "memory");
+		} else {
+			asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+		}
+		half_sync(half);
+		// the index after next arrives during the products
+		int w2 = nW;
+		if (lt == 0 && wn < nW) w2 = atomicAdd(ctr, 1);
+		phase2_item(st + 3 * cur, it, half, lt, ro, nb, kp, dst, V);
+		if (lt == 0) sh.next[half] = w2;
+		half_sync(half);  // the stage is free for the item after next
+		it = nx;
+		w = wn;
+		wn = sh.next[half];
+		cur ^= 1;
+	}
 }
 
 // Buffers: A_r lives in bufs[(r + 1) % 3] (A_{-1} = the input in A0); Q_r in
@@ -573,7 +794,7 @@ __global__ void __launch_bounds__(kThreads, 1) bjacobi_kernel(double2* A0, doubl
 	const int np = nb / 2;
 	const int rounds = nb - 1;
 	const int nrb = kp / MS;
-	const int nW = np * (np - 1) + nrb * np;
+	const int nW = np * (np - 1) / 2 + nrb * np;
 	double2* const bufs[3] = {A0, A1, A2};
 	const size_t qstride = (size_t)np * MS * MS;
 	// CTAs [0, p1) take phase 1 items, the rest phase 2 items (all CTAs take
@@ -612,21 +833,7 @@ __global__ void __launch_bounds__(kThreads, 1) bjacobi_kernel(double2* A0, doubl
 			const int ro = (int)((t - 1) % rounds);
 			const double2* src = bufs[(t + 2) % 3];
 			double2* dst = bufs[t % 3];
-			// items handed out by the round's counter; the next index is fetched
-			// while the current item is processed
-			const int half = tid / (kThreads / 2), lt = tid & (kThreads / 2 - 1);
-			int* ctr = p2ctr + ((t - 1) & 3);
-			if (lt == 0) sh.next[half] = atomicAdd(ctr, 1);
-			half_sync(half);
-			int w = sh.next[half];
-			while (w < nW) {
-				int wn = 0;
-				if (lt == 0) wn = atomicAdd(ctr, 1);
-				phase2_item(sh, half, w, ro, nb, np, kp, src, dst, V, Qbuf + ((t + 1) & 1) * qstride);
-				if (lt == 0) sh.next[half] = wn;
-				half_sync(half);
-				w = sh.next[half];
-			}
+			phase2(sh, ro, nb, np, nW, kp, src, dst, V, Qbuf + ((t + 1) & 1) * qstride, p2ctr + ((t - 1) & 3));
 		}
 		const bool sweep_end = do_p1 && (t % rounds == rounds - 1);
 		if (sweep_end && tid == 0) {
@@ -671,7 +878,10 @@ cudaError_t launch_bjacobi(double2* A0, double2* A1, double2* A2, double2* V, do
 	e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, bjacobi_kernel, kThreads, smem);
 	if (e != cudaSuccess) return e;
 	if (per_sm < 1) return cudaErrorLaunchOutOfResources;
-	const int blocks = num_sms * std::min(per_sm, 1);
+	// one CTA per phase-1 pair and one per two phase-2 items, at most one per SM:
+	// the grid barrier of a small problem spans few CTAs
+	const int np = kp / MS, nW = np * (np - 1) / 2 + np * np;
+	const int blocks = std::min(num_sms, np + (nW + 1) / 2);
 	double tol = 1e-15;
 	if (!(tau_final > 0.0)) tau_final = kTauFinal;
 	unsigned long long* tmax = reinterpret_cast<unsigned long long*>(counters + jacobi_tmax_offset(max_sweeps));

@@ -58,20 +58,20 @@ struct EigStatus {
 };
 
 struct JacobiWork {
-	double2* A0;      // k x k working matrix (input S, overwritten)
-	double2* A1;      // k x k second buffer
-	double2* V;       // k x k eigenvectors (columns)
+	double2* A0;      // kp x kp working matrix (kp = jacobi_kp(k))
+	double2* A1;      // kp x kp second buffer
+	double2* V;       // kp x kp eigenvectors (columns)
 	double* evals;    // k
 	int* perm;        // k
 	int* counters;    // jacobi_counter_ints(max_sweeps) ints
 	int max_sweeps;
-	double2* Qbuf = nullptr;  // block Jacobi unitaries (bjacobi_qbuf_elems); null: scalar Jacobi only
-	double2* A2 = nullptr;    // third kp x kp buffer of the block path (required with Qbuf)
+	double2* Qbuf = nullptr;  // block unitaries of two rounds (bjacobi_qbuf_elems)
+	double2* A2 = nullptr;    // kp x kp third buffer
 	// Stop after a sweep whose largest rotation tangent is below tau_final;
 	// 0 selects the FP64 default of the kernel. The remaining off-diagonal
 	// elements are then of order tau_final^2 relative to the eigenvalue gaps.
 	double tau_final = 0.0;
-	// FP32 block path (launch_bjacobi32): set, with k >= kBlockJacobiMinK, the
+	// FP32 path (launch_bjacobi32): set, with k >= kBlockJacobi32MinK, the
 	// solve runs in single precision on these kp x kp buffers and widens its
 	// result into A0 (diagonal) and V. They may alias A1, A2 and Qbuf, which
 	// that path does not use otherwise; none may alias A0 or V.
@@ -87,14 +87,16 @@ struct JacobiWork {
 	bool full_result = false;
 };
 
-// Smallest k solved by block Jacobi (when JacobiWork::Qbuf is set).
-constexpr int kBlockJacobiMinK = 256;
-// Padded dimension of the block path (multiple of 32) and its Q buffer size
+// Smallest k of FP32 states solved in single precision; below it the FP64
+// solver runs (a smaller overlap is not worth the lower precision: the whole
+// FP64 solve takes well under a millisecond).
+constexpr int kBlockJacobi32MinK = 256;
+// Padded dimension of the eigensolvers (multiple of 32) and their Q buffer size
 // (the unitaries of two rounds).
 int bjacobi_padded(int k);
 size_t bjacobi_qbuf_elems(int k);
-// Padded dimension the eigensolver uses for (w, k); A0/A1/V are kp x kp.
-int jacobi_kp(const JacobiWork& w, int k);
+// Row stride of the eigensolver's matrices: A0, A1, A2 and V are kp x kp.
+int jacobi_kp(int k);
 cudaError_t launch_bjacobi(double2* A0, double2* A1, double2* A2, double2* V, double2* Qbuf, int kp,
 		int max_sweeps, double tau_final, int* counters, int num_sms, cudaStream_t s);
 // Single-precision block Jacobi of S (k x k, FP64) on w.f32; leaves the
@@ -103,13 +105,13 @@ cudaError_t launch_bjacobi(double2* A0, double2* A1, double2* A2, double2* V, do
 cudaError_t launch_bjacobi32(const double2* S, int k, JacobiWork& w, int num_sms, cudaStream_t s);
 
 // Eigen-decomposition of the Hermitian S (k x k, row-major, full storage) by
-// parallel cyclic Jacobi, then W[:, n] = V[:, p(n)] / sqrt(l_n) with l
+// block Jacobi, then W[:, n] = V[:, p(n)] / sqrt(l_n) with l
 // ascending, and the eigenvalue checks of stateset.cpp:158-173. S is
 // consumed. Returns a CUDA error code of the launches (status goes to *st).
 cudaError_t launch_eigensolve(double2* S, int k, JacobiWork& w, double2* W, EigStatus* st, int num_sms,
 		cudaStream_t s);
 // Eigenvalues (ascending, w.evals), permutation (w.perm) and eigenvectors
-// (columns of w.V, kp x kp with kp = k rounded up to even) without the
+// (columns of w.V, kp x kp with kp = jacobi_kp(k)) without the
 // overlap checks unless check != 0; check 2 also accepts a solve that ended
 // at w.max_sweeps without converging (sweeps reported as w.max_sweeps).
 cudaError_t launch_eigh(double2* S, int k, JacobiWork& w, EigStatus* st, int num_sms, cudaStream_t s, int check);

@@ -775,15 +775,15 @@ long long itp2d_ctx_footprint(int sx, int sy, int num_states, int boundary, doub
 	const int npairs = nt * (nt + 1) / 2;
 	const int nsplit = overlap_splits(num_states, G, sms);
 	const int parts = std::max(nsplit, tc_overlap_splits(num_states, G, sms));
-	const long long kp = std::max(bjacobi_padded(num_states), (num_states + 1) & ~1);
+	const long long kp = jacobi_kp(num_states);
 	// tensor-core scratch of the FP32 form: W^T planes, pre-split states for
 	// the overlap and the rotation (counted whenever the size can use them)
 	b += (2 + parts) * k * k * 16 + (tc_supported(num_states, G) ? (long long)(tc_wsplit_bytes(num_states) +
 	                                                                           tc_rows_bytes(num_states, G) +
 	                                                                           tc_cols_bytes(num_states, G))
 	                                                             : 0);
-	b += (num_states >= kBlockJacobiMinK ? 4 : 3) * kp * kp * 16 + npairs * 8;
-	if (num_states >= kBlockJacobiMinK) b += (long long)bjacobi_qbuf_elems(num_states) * 16;
+	b += 4 * kp * kp * 16 + npairs * 8;
+	b += (long long)bjacobi_qbuf_elems(num_states) * 16;
 	b += k * std::max(sx, sy) * 5 * 8 * (dm ? 2 : 1) + 5 * k * 8 + 16 * k;
 	// tables: three potential exponentials and a kinetic table per member, the
 	// energy tables, and the line plans (twiddles)
@@ -833,7 +833,7 @@ int itp2d_ctx_create(int sx, int sy, double dx, int num_states, int boundary, do
 	const int nt = overlap_tiles(k);
 	c->npairs = nt * (nt + 1) / 2;
 	c->nsplit = overlap_splits(k, c->G, c->num_sms);
-	const int kp = std::max(bjacobi_padded(k), (k + 1) & ~1);  // covers the scalar and block layouts
+	const int kp = jacobi_kp(k);
 	if (e == cudaSuccess) c->S = (double2*)dalloc(c, (size_t)k * k * sizeof(double2), &e);
 	c->tc_nsplit = tc_overlap_splits(k, c->G, c->num_sms);
 	const int parts = std::max(c->nsplit, c->tc_nsplit);
@@ -847,10 +847,8 @@ int itp2d_ctx_create(int sx, int sy, double dx, int num_states, int boundary, do
 	if (e == cudaSuccess) c->jw.A0 = (double2*)dalloc(c, (size_t)kp * kp * sizeof(double2), &e);
 	if (e == cudaSuccess) c->jw.A1 = (double2*)dalloc(c, (size_t)kp * kp * sizeof(double2), &e);
 	if (e == cudaSuccess) c->jw.V = (double2*)dalloc(c, (size_t)kp * kp * sizeof(double2), &e);
-	if (e == cudaSuccess && k >= kBlockJacobiMinK)
-		c->jw.Qbuf = (double2*)dalloc(c, bjacobi_qbuf_elems(k) * sizeof(double2), &e);
-	if (e == cudaSuccess && k >= kBlockJacobiMinK)
-		c->jw.A2 = (double2*)dalloc(c, (size_t)kp * kp * sizeof(double2), &e);
+	if (e == cudaSuccess) c->jw.Qbuf = (double2*)dalloc(c, bjacobi_qbuf_elems(k) * sizeof(double2), &e);
+	if (e == cudaSuccess) c->jw.A2 = (double2*)dalloc(c, (size_t)kp * kp * sizeof(double2), &e);
 	if (e == cudaSuccess) c->jw.evals = (double*)dalloc(c, (size_t)k * sizeof(double), &e);
 	if (e == cudaSuccess) c->jw.perm = (int*)dalloc(c, (size_t)k * sizeof(int), &e);
 	if (e == cudaSuccess) c->jw.counters = (int*)dalloc(c, jacobi_counters(c->jw.max_sweeps) * sizeof(int), &e);
@@ -1306,7 +1304,7 @@ static int cholesky_w(itp2d_ctx* c, int* bad_index, double* bad_value) {
 static int capped_w(itp2d_ctx* c, bool* done, int* sweeps, int* bad_index, double* bad_value) {
 	*done = false;
 	JacobiWork& w = c->jw;
-	if (!w.f32.A0 || c->k < kBlockJacobiMinK) return ITP2D_OK;
+	if (!w.f32.A0 || c->k < kBlockJacobi32MinK) return ITP2D_OK;
 	const int ms = w.max_sweeps;
 	w.max_sweeps = c->fp32_sweep_cap;
 	w.full_result = true;
@@ -1412,7 +1410,7 @@ int itp2d_orthonormalize(itp2d_ctx* c, int algo, int* bad_index, double* bad_val
 		// FP32 states also solve in FP32, on views of the FP64 buffers the block
 		// path leaves free (A1 holds two FP32 matrices, A2 two more)
 		c->jw.f32 = {};
-		if (!f64 && c->jw.Qbuf && c->jw.A2) {
+		if (!f64 && c->k >= kBlockJacobi32MinK) {
 			const size_t kp2 = (size_t)bjacobi_padded(c->k) * bjacobi_padded(c->k);
 			c->jw.f32.A0 = (float2*)c->jw.A1;
 			c->jw.f32.A1 = c->jw.f32.A0 + kp2;
@@ -1579,7 +1577,7 @@ long long itp2d_precision_sweeps(itp2d_ctx* c, int precision) {
 int itp2d_hermitian_eigensolve(int n, const double* A, double* evals, double* evecs) {
 	if (n < 1 || !A || !evals || !evecs) return ITP2D_E_INVALID;
 	CoopUser user;
-	const int kp = std::max(bjacobi_padded(n), (n + 1) & ~1);
+	const int kp = jacobi_kp(n);
 	std::vector<double2> S((size_t)n * n);
 	for (int i = 0; i < n; i++)
 		for (int j = i; j < n; j++) {
@@ -1603,15 +1601,15 @@ int itp2d_hermitian_eigensolve(int n, const double* A, double* evals, double* ev
 	w.A0 = (double2*)al((size_t)kp * kp * sizeof(double2));
 	w.A1 = (double2*)al((size_t)kp * kp * sizeof(double2));
 	w.V = (double2*)al((size_t)kp * kp * sizeof(double2));
-	if (n >= kBlockJacobiMinK) w.Qbuf = (double2*)al(bjacobi_qbuf_elems(n) * sizeof(double2));
-	if (n >= kBlockJacobiMinK) w.A2 = (double2*)al((size_t)kp * kp * sizeof(double2));
+	w.Qbuf = (double2*)al(bjacobi_qbuf_elems(n) * sizeof(double2));
+	w.A2 = (double2*)al((size_t)kp * kp * sizeof(double2));
 	w.evals = (double*)al((size_t)n * sizeof(double));
 	w.perm = (int*)al((size_t)n * sizeof(int));
 	w.counters = (int*)al(jacobi_counters(w.max_sweeps) * sizeof(int));
 	EigStatus* dst = (EigStatus*)al(sizeof(EigStatus));
 	int status = ITP2D_OK;
-	if (!dS || !w.A0 || !w.A1 || !w.V || !w.evals || !w.perm || !w.counters || !dst ||
-			(n >= kBlockJacobiMinK && (!w.Qbuf || !w.A2)))
+	if (!dS || !w.A0 || !w.A1 || !w.V || !w.evals || !w.perm || !w.counters || !dst || !w.Qbuf ||
+			!w.A2)
 		status = ITP2D_E_OOM;
 	std::vector<double2> V;
 	std::vector<int> perm(n);
@@ -1629,7 +1627,7 @@ int itp2d_hermitian_eigensolve(int n, const double* A, double* evals, double* ev
 		if (status == ITP2D_OK && hs.status != ITP2D_OK) status = hs.status;
 	}
 	if (status == ITP2D_OK) {
-		const int jkp = jacobi_kp(w, n);
+		const int jkp = jacobi_kp(n);
 		for (int m = 0; m < n; m++)
 			for (int i = 0; i < n; i++) {
 				const double2 v = V[(size_t)i * jkp + perm[m]];

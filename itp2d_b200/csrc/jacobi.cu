@@ -1,261 +1,24 @@
 // Hermitian eigen-decomposition of the k x k overlap matrix on the GPU.
 //
 // Replaces EigenSolver::solve (ZHEEV, eigensolver.hpp:80-84) and the checks
-// and scaling of StateSet::orthonormalize (stateset.cpp:155-176). Method:
-// parallel cyclic two-sided Jacobi. Each round applies kp/2 disjoint complex
-// plane rotations J_pq (round-robin "circle" pairing, every pair once per
-// sweep), A <- J^H A J and V <- V J, with A double-buffered so a round needs
-// one grid-wide barrier. Rotation angles follow the classical Jacobi
-// formulas (tan of the smaller angle), lifted to the Hermitian case by the
-// phase of A_pq. A rotation is skipped when |A_pq| <= tol sqrt(|A_pp A_qq|),
-// which gives the high relative accuracy Jacobi is known for on positive
-// definite matrices; a sweep without rotations ends the iteration.
+// and scaling of StateSet::orthonormalize (stateset.cpp:155-176): the block
+// Jacobi iteration of bjacobi.cu (FP64, every k) or bjacobi32.cu (FP32 states
+// of kBlockJacobi32MinK and more), then the steps of this file: unit columns,
+// the ascending sort with the reference's checks, and W = V l^{-1/2}.
+//
+// FP64 block Jacobi serves small k too: a sweep of k = 200 takes 13 grid-wide
+// rounds of 16 x 16 rotations in shared memory, where one grid-wide round per
+// k/2 rotations (scalar cyclic Jacobi, 199 rounds of 8.8 us each) took 17.5 ms
+// per eigensolve.
 #include <atomic>
 #include <mutex>
-
-#include <cooperative_groups.h>
 
 #include "contract.cuh"
 #include "../../include/itp2d_gpu.h"
 
-namespace cg = cooperative_groups;
-
 namespace itp2d {
 
 namespace {
-
-constexpr int TP = 16;        // pair slots per tile side
-constexpr int kVRows = 32;    // V rows per work item
-constexpr int kThreads = 256;
-
-struct Rot {
-	double c, s, er, ei;  // J = [[c, s e], [-s conj(e), c]], e = er + i ei
-	double ap, aq;        // rotated diagonal
-	double t;             // |tan| of the rotation angle (0 when skipped)
-	int rotated;
-};
-
-__device__ __forceinline__ int player(int pos, int r, int kp) {
-	return pos == 0 ? 0 : ((pos - 1 + r) % (kp - 1)) + 1;
-}
-
-__device__ __forceinline__ double2 ldA(const double2* A, long long idx) { return __ldcg(A + idx); }
-
-__device__ void make_rot(Rot& R, const double2* A, int kp, int slot, int r, double tol) {
-	const int p = player(slot, r, kp);
-	const int q = player(kp - 1 - slot, r, kp);
-	const double a = ldA(A, (long long)p * kp + p).x;
-	const double b = ldA(A, (long long)q * kp + q).x;
-	const double2 c = ldA(A, (long long)p * kp + q);
-	const double cabs = hypot(c.x, c.y);
-	R.c = 1.0; R.s = 0.0; R.er = 1.0; R.ei = 0.0; R.ap = a; R.aq = b; R.t = 0.0; R.rotated = 0;
-	if (cabs > 0.0 && cabs > tol * sqrt(fabs(a) * fabs(b))) {
-		const double th = (b - a) / (2.0 * cabs);
-		const double ath = fabs(th);
-		const double t = (ath > 1e150) ? 0.5 / ath : 1.0 / (ath + sqrt(th * th + 1.0));
-		if (t != 0.0) {
-			R.c = 1.0 / sqrt(t * t + 1.0);
-			R.s = (th < 0 ? -t : t) * R.c;
-			R.er = c.x / cabs;
-			R.ei = c.y / cabs;
-			R.ap = a - (th < 0 ? -t : t) * cabs;
-			R.aq = b + (th < 0 ? -t : t) * cabs;
-			R.t = t;
-			R.rotated = 1;
-		}
-	}
-}
-
-__device__ __forceinline__ double2 cm(double2 a, double2 b) {
-	return make_double2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
-}
-__device__ __forceinline__ double2 cadd2(double2 a, double2 b) { return make_double2(a.x + b.x, a.y + b.y); }
-__device__ __forceinline__ double2 csc(double2 a, double s) { return make_double2(a.x * s, a.y * s); }
-__device__ __forceinline__ double2 cconj(double2 a) { return make_double2(a.x, -a.y); }
-
-// Rows of J^H X for J = [[c, s e], [-s conj(e), c]], written as corrections
-// of the old values (tau = s / (1 + c)), which keeps small rotations accurate.
-__device__ __forceinline__ void rot_rows(const Rot& R, double2 xp, double2 xq, double2& yp, double2& yq) {
-	const double tau = R.s / (1.0 + R.c);
-	const double2 e = make_double2(R.er, R.ei);
-	yp = cadd2(xp, csc(cadd2(cm(e, xq), csc(xp, tau)), -R.s));
-	yq = cadd2(xq, csc(cadd2(cm(cconj(e), xp), csc(xq, -tau)), R.s));
-}
-
-// Columns of X J in the same correction form.
-__device__ __forceinline__ void rot_cols(const Rot& C, double2 xs, double2 xt, double2& ys, double2& yt) {
-	const double tau = C.s / (1.0 + C.c);
-	const double2 e = make_double2(C.er, C.ei);
-	ys = cadd2(xs, csc(cadd2(cm(cconj(e), xt), csc(xs, tau)), -C.s));
-	yt = cadd2(xt, csc(cadd2(cm(e, xs), csc(xt, -tau)), C.s));
-}
-
-constexpr int kItems = 2;  // work items per CTA between two CTA barriers
-
-// Tangent below which a sweep is final: the next sweep could only change
-// off-diagonal elements by O(k tau^2) relative to the eigenvalue gaps.
-constexpr double kTauFinal = 1e-10;
-
-// One cooperative launch = the whole eigensolve. Per round, each CTA takes up
-// to kItems work items (an A tile of TP x TP pair blocks, or a V tile of
-// kVRows rows x TP pairs), issues all of their global loads together with the
-// loads of the rotation inputs, then applies the rotations after one CTA
-// barrier; the round ends with one grid barrier.
-__global__ void __launch_bounds__(kThreads) jacobi_kernel(double2* A0, double2* A1, double2* V, int kp,
-		int max_sweeps, double tol, double tau_final, int* counters, unsigned long long* tmax) {
-	cg::grid_group grid = cg::this_grid();
-	__shared__ Rot rr[kItems][TP];
-	__shared__ Rot rc[kItems][TP];
-	__shared__ int s_cnt;                 // rotations applied by this CTA in the sweep
-	__shared__ unsigned long long s_tmax;  // largest tangent (bit pattern of a non-negative double)
-	const int tid = threadIdx.x;
-	if (tid == 0) {
-		s_cnt = 0;
-		s_tmax = 0ULL;
-	}
-	__syncthreads();
-	const int np = kp / 2;
-	const int nt = (np + TP - 1) / TP;
-	const int nA = nt * nt;
-	const int nVr = (kp + kVRows - 1) / kVRows;
-	const int nW = nA + nVr * nt;
-	double2* Acur = A0;
-	double2* Anext = A1;
-	int sweep = 0;
-	bool converged = false;
-	for (; sweep < max_sweeps && !converged; sweep++) {
-		for (int r = 0; r < kp - 1; r++) {
-			for (int w0 = blockIdx.x * kItems; w0 < nW; w0 += gridDim.x * kItems) {
-				double2 x[kItems][4];
-				// phase 1: rotation set-up and all loads
-#pragma unroll
-				for (int it = 0; it < kItems; it++) {
-					const int w = w0 + it;
-					if (w >= nW) break;
-					if (w < nA) {
-						const int TI = w / nt, TJ = w % nt;
-						if (tid < TP) {
-							const int sl = TI * TP + tid;
-							if (sl < np) make_rot(rr[it][tid], Acur, kp, sl, r, tol);
-						} else if (tid < 2 * TP) {
-							const int sl = TJ * TP + tid - TP;
-							if (sl < np) make_rot(rc[it][tid - TP], Acur, kp, sl, r, tol);
-						}
-						const int sa = TI * TP + tid / TP, sb = TJ * TP + tid % TP;
-						if (sa < np && sb < np) {
-							const int p = player(sa, r, kp), q = player(kp - 1 - sa, r, kp);
-							const int s2 = player(sb, r, kp), t2 = player(kp - 1 - sb, r, kp);
-							if (sa == sb) {
-								x[it][0] = ldA(Acur, (long long)p * kp + q);
-								x[it][1] = ldA(Acur, (long long)q * kp + p);
-							} else {
-								x[it][0] = ldA(Acur, (long long)p * kp + s2);
-								x[it][1] = ldA(Acur, (long long)p * kp + t2);
-								x[it][2] = ldA(Acur, (long long)q * kp + s2);
-								x[it][3] = ldA(Acur, (long long)q * kp + t2);
-							}
-						}
-					} else {
-						const int v = w - nA;
-						const int RC = v / nt, TJ = v % nt;
-						if (tid < TP) {
-							const int sl = TJ * TP + tid;
-							if (sl < np) make_rot(rc[it][tid], Acur, kp, sl, r, tol);
-						}
-#pragma unroll
-						for (int h = 0; h < 2; h++) {
-							const int e = tid + h * kThreads;
-							const int i = RC * kVRows + e / TP, sb = TJ * TP + e % TP;
-							if (i < kp && sb < np) {
-								const int s2 = player(sb, r, kp), t2 = player(kp - 1 - sb, r, kp);
-								x[it][2 * h] = ldA(V, (long long)i * kp + s2);
-								x[it][2 * h + 1] = ldA(V, (long long)i * kp + t2);
-							}
-						}
-					}
-				}
-				__syncthreads();
-				// phase 2: apply
-#pragma unroll
-				for (int it = 0; it < kItems; it++) {
-					const int w = w0 + it;
-					if (w >= nW) break;
-					if (w < nA) {
-						const int TI = w / nt, TJ = w % nt;
-						const int a = tid / TP, b = tid % TP;
-						const int sa = TI * TP + a, sb = TJ * TP + b;
-						if (sa >= np || sb >= np) continue;
-						const Rot& R = rr[it][a];
-						const Rot& C = rc[it][b];
-						const int p = player(sa, r, kp), q = player(kp - 1 - sa, r, kp);
-						if (sa == sb) {
-							Anext[(long long)p * kp + p] = make_double2(R.ap, 0.0);
-							Anext[(long long)q * kp + q] = make_double2(R.aq, 0.0);
-							if (R.rotated) {
-								Anext[(long long)p * kp + q] = make_double2(0.0, 0.0);
-								Anext[(long long)q * kp + p] = make_double2(0.0, 0.0);
-								atomicAdd(&s_cnt, 1);
-								atomicMax(&s_tmax, (unsigned long long)__double_as_longlong(R.t));
-							} else {
-								Anext[(long long)p * kp + q] = x[it][0];
-								Anext[(long long)q * kp + p] = x[it][1];
-							}
-							continue;
-						}
-						const int s2 = player(sb, r, kp), t2 = player(kp - 1 - sb, r, kp);
-						double2 y1s, y1t, y2s, y2t, o1, o2;
-						rot_rows(R, x[it][0], x[it][2], y1s, y2s);
-						rot_rows(R, x[it][1], x[it][3], y1t, y2t);
-						rot_cols(C, y1s, y1t, o1, o2);
-						Anext[(long long)p * kp + s2] = o1;
-						Anext[(long long)p * kp + t2] = o2;
-						rot_cols(C, y2s, y2t, o1, o2);
-						Anext[(long long)q * kp + s2] = o1;
-						Anext[(long long)q * kp + t2] = o2;
-					} else {
-						const int v = w - nA;
-						const int RC = v / nt, TJ = v % nt;
-#pragma unroll
-						for (int h = 0; h < 2; h++) {
-							const int e = tid + h * kThreads;
-							const int i = RC * kVRows + e / TP, b = e % TP, sb = TJ * TP + b;
-							if (i >= kp || sb >= np) continue;
-							const Rot& C = rc[it][b];
-							if (!C.rotated) continue;
-							const int s2 = player(sb, r, kp), t2 = player(kp - 1 - sb, r, kp);
-							double2 ns, nt2;
-							rot_cols(C, x[it][2 * h], x[it][2 * h + 1], ns, nt2);
-							V[(long long)i * kp + s2] = ns;
-							V[(long long)i * kp + t2] = nt2;
-						}
-					}
-				}
-				__syncthreads();
-			}
-			grid.sync();
-			double2* tmp = Acur;
-			Acur = Anext;
-			Anext = tmp;
-		}
-		// one global update per CTA and sweep, then a grid barrier so every CTA
-		// reads the final totals
-		if (tid == 0) {
-			if (s_cnt) atomicAdd(&counters[sweep], s_cnt);
-			if (s_tmax) atomicMax(&tmax[sweep], s_tmax);
-			s_cnt = 0;
-			s_tmax = 0ULL;
-		}
-		grid.sync();
-		// uniform across the grid: everything below reads values final after grid.sync
-		const int cnt = *((volatile int*)&counters[sweep]);
-		const double tm = __longlong_as_double((long long)*((volatile unsigned long long*)&tmax[sweep]));
-		if (cnt == 0 || tm < tau_final) converged = true;
-	}
-	if (blockIdx.x == 0 && threadIdx.x == 0) {
-		counters[max_sweeps] = converged ? sweep : -1;   // sweeps used, -1: no convergence
-		counters[max_sweeps + 1] = (Acur == A0) ? 0 : 1;  // buffer holding the result
-	}
-}
 
 // Copy S (k x k) into the padded kp x kp work matrix; V = I.
 __global__ void jacobi_init_kernel(const double2* __restrict__ S, int k, int kp, double2* A, double2* V) {
@@ -440,7 +203,7 @@ cudaError_t launch_eigensolve(double2* S, int k, JacobiWork& w, double2* W, EigS
 	cudaError_t e = launch_eigh(S, k, w, st, num_sms, s, 1);
 	if (e != cudaSuccess) return e;
 	const long long n2 = (long long)k * k;
-	const int kp = jacobi_kp(w, k);
+	const int kp = jacobi_kp(k);
 	build_w_kernel<<<(unsigned)std::min<long long>((n2 + 255) / 256, 4096), 256, 0, s>>>(w.V, k, kp, w.evals,
 			w.perm, W);
 	return cudaGetLastError();
@@ -450,7 +213,7 @@ cudaError_t launch_ritz(double2* H, int k, JacobiWork& w, double2* W, EigStatus*
 	cudaError_t e = launch_eigh(H, k, w, st, num_sms, s, 0);
 	if (e != cudaSuccess) return e;
 	const long long n2 = (long long)k * k;
-	ritz_w_kernel<<<(unsigned)std::min<long long>((n2 + 255) / 256, 4096), 256, 0, s>>>(w.V, k, jacobi_kp(w, k),
+	ritz_w_kernel<<<(unsigned)std::min<long long>((n2 + 255) / 256, 4096), 256, 0, s>>>(w.V, k, jacobi_kp(k),
 			w.perm, W);
 	return cudaGetLastError();
 }
@@ -458,16 +221,14 @@ cudaError_t launch_ritz(double2* H, int k, JacobiWork& w, double2* W, EigStatus*
 cudaError_t launch_eig_cholesky_prep(const JacobiWork& w, int k, double2* S_out, double2* VT, cudaStream_t s) {
 	const long long n2 = (long long)k * k;
 	eig_cholesky_prep_kernel<<<(unsigned)std::min<long long>((n2 + 255) / 256, 4096), 256, 0, s>>>(w.A0, w.A1, w.A2,
-			w.V, w.perm, w.counters, w.max_sweeps, k, jacobi_kp(w, k), S_out, VT);
+			w.V, w.perm, w.counters, w.max_sweeps, k, jacobi_kp(k), S_out, VT);
 	return cudaGetLastError();
 }
 
-int jacobi_kp(const JacobiWork& w, int k) {
-	return (w.Qbuf && w.A2 && k >= kBlockJacobiMinK) ? bjacobi_padded(k) : ((k + 1) & ~1);
-}
+int jacobi_kp(int k) { return bjacobi_padded(k); }
 
 cudaError_t launch_eigh(double2* S, int k, JacobiWork& w, EigStatus* st, int num_sms, cudaStream_t s, int check) {
-	const int kp = jacobi_kp(w, k);
+	const int kp = jacobi_kp(k);
 	const long long n = (long long)kp * kp;
 	cudaError_t e = cudaMemsetAsync(w.counters, 0, jacobi_counters(w.max_sweeps) * sizeof(int), s);
 	if (e != cudaSuccess) return e;
@@ -475,35 +236,14 @@ cudaError_t launch_eigh(double2* S, int k, JacobiWork& w, EigStatus* st, int num
 	// held until the kernel below has finished
 	std::unique_lock<std::mutex> serial;
 	if (g_coop_users.load() > 1) serial = std::unique_lock<std::mutex>(g_coop_mu);
-	if (w.f32.A0 && w.Qbuf && w.A2 && k >= kBlockJacobiMinK) {
+	if (w.f32.A0 && k >= kBlockJacobi32MinK) {
 		e = launch_bjacobi32(S, k, w, num_sms, s);
-		if (e != cudaSuccess) return e;
-	} else if (w.Qbuf && w.A2 && k >= kBlockJacobiMinK) {
-		jacobi_init_kernel<<<(unsigned)std::min<long long>((n + 255) / 256, 4096), 256, 0, s>>>(S, k, kp, w.A0,
-				w.V);
-		e = launch_bjacobi(w.A0, w.A1, w.A2, w.V, w.Qbuf, kp, w.max_sweeps, w.tau_final, w.counters, num_sms, s);
-		if (e != cudaSuccess) return e;
 	} else {
 		jacobi_init_kernel<<<(unsigned)std::min<long long>((n + 255) / 256, 4096), 256, 0, s>>>(S, k, kp, w.A0,
 				w.V);
-		int per_sm = 0;
-		e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, jacobi_kernel, kThreads, 0);
-		if (e != cudaSuccess) return e;
-		if (per_sm < 1) return cudaErrorLaunchOutOfResources;
-		const int np = kp / 2;
-		const int nt = (np + TP - 1) / TP;
-		const int nW = nt * nt + ((kp + kVRows - 1) / kVRows) * nt;
-		int blocks = std::min(num_sms * std::min(per_sm, 2), (nW + kItems - 1) / kItems);
-		if (blocks < 1) blocks = 1;
-		double tol = 1e-15;
-		double tau_final = w.tau_final > 0.0 ? w.tau_final : kTauFinal;
-		int ms = w.max_sweeps;
-		int kpv = kp;
-		unsigned long long* tmax = reinterpret_cast<unsigned long long*>(w.counters + jacobi_tmax_offset(ms));
-		void* args[] = {&w.A0, &w.A1, &w.V, (void*)&kpv, &ms, &tol, &tau_final, &w.counters, &tmax};
-		e = cudaLaunchCooperativeKernel((void*)jacobi_kernel, dim3(blocks), dim3(kThreads), args, 0, s);
-		if (e != cudaSuccess) return e;
+		e = launch_bjacobi(w.A0, w.A1, w.A2, w.V, w.Qbuf, kp, w.max_sweeps, w.tau_final, w.counters, num_sms, s);
 	}
+	if (e != cudaSuccess) return e;
 	if (serial.owns_lock()) {
 		e = cudaStreamSynchronize(s);
 		serial.unlock();

@@ -11,7 +11,7 @@
 // nothing, on the device or on the host.
 //
 // The array holds at most ITP2D_NOALLOC_MAX_N x ITP2D_NOALLOC_MAX_N matrices
-// (about 1.6 MB in total) and stays resident on every GPU that loads the
+// (about 2 MB in total) and stays resident on every GPU that loads the
 // library until the process exits. Every call uses the same array, so calls
 // that overlap on the GPU (from several host threads, or on several streams)
 // race and must be serialised by the caller. Every call looks up the array's
@@ -32,13 +32,18 @@ constexpr int kMaxSweeps = 60;
 constexpr size_t kAlign = 256;
 constexpr size_t align_up(size_t b) { return (b + kAlign - 1) / kAlign * kAlign; }
 constexpr size_t kMatBytes = align_up((size_t)kMaxN * kMaxN * sizeof(double2));
-// input, S, A0, A1, V, eigenvector output, eigenvalues, permutation, counters, status
+static_assert(kMaxN % 32 == 0, "the solver pads its matrices to a multiple of 32");
+// block unitaries of two rounds: 2 (kMaxN / 32) of 32 x 32
+constexpr size_t kQbufBytes = align_up((size_t)2 * (kMaxN / 32) * 32 * 32 * sizeof(double2));
+// input, S, A0, A1, A2, V, Q, eigenvector output, eigenvalues, permutation, counters, status
 constexpr size_t kOffIn = 0;
 constexpr size_t kOffS = kOffIn + kMatBytes;
 constexpr size_t kOffA0 = kOffS + kMatBytes;
 constexpr size_t kOffA1 = kOffA0 + kMatBytes;
-constexpr size_t kOffV = kOffA1 + kMatBytes;
-constexpr size_t kOffVec = kOffV + kMatBytes;
+constexpr size_t kOffA2 = kOffA1 + kMatBytes;
+constexpr size_t kOffV = kOffA2 + kMatBytes;
+constexpr size_t kOffQ = kOffV + kMatBytes;
+constexpr size_t kOffVec = kOffQ + kQbufBytes;
 constexpr size_t kOffEval = kOffVec + kMatBytes;
 constexpr size_t kOffPerm = kOffEval + align_up(kMaxN * sizeof(double));
 constexpr size_t kOffCnt = kOffPerm + align_up(kMaxN * sizeof(int));
@@ -106,12 +111,14 @@ extern "C" int itp2d_hermitian_eigensolve_noalloc(int n, const double* A, double
 	JacobiWork w;
 	w.A0 = reinterpret_cast<double2*>(base + kOffA0);
 	w.A1 = reinterpret_cast<double2*>(base + kOffA1);
+	w.A2 = reinterpret_cast<double2*>(base + kOffA2);
 	w.V = reinterpret_cast<double2*>(base + kOffV);
+	w.Qbuf = reinterpret_cast<double2*>(base + kOffQ);
 	w.evals = reinterpret_cast<double*>(base + kOffEval);
 	w.perm = reinterpret_cast<int*>(base + kOffPerm);
 	w.counters = reinterpret_cast<int*>(base + kOffCnt);  // cleared by launch_eigh on every call
 	w.max_sweeps = kMaxSweeps;
-	const int kp = (n + 1) & ~1;
+	const int kp = itp2d::jacobi_kp(n);
 	const int nn = n * n;
 	cudaError_t e = cudaMemcpy(in, A, (size_t)nn * sizeof(double2), cudaMemcpyHostToDevice);
 	if (e != cudaSuccess) return status_of(e);
