@@ -239,7 +239,7 @@ class Context:
                "itp2d_set_fp32_orthonormalization")
 
     def set_column_variant(self, variant):
-        """Column pass of 256/512-point lines: COL_SMEM, COL_TMA, or -1 (tuned)."""
+        """Names the column pass: COL_SMEM, COL_TMA (the same pass), or -1 (default)."""
         _check(lib().itp2d_set_column_variant(self.h, int(variant)), "itp2d_set_column_variant")
 
     @property

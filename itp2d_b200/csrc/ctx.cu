@@ -10,8 +10,6 @@
 #include <cmath>
 #include <cstdio>
 #include <cstring>
-#include <map>
-#include <tuple>
 #include <mutex>
 #include <new>
 #include <string>
@@ -132,9 +130,6 @@ struct itp2d_ctx {
 	long long ortho_calls[3] = {0, 0, 0};  // canonical, Lowdin, Cholesky
 	long long ritz_calls = 0;              // Rayleigh-Ritz steps
 	long long tri_rot[2] = {0, 0};         // rotations by an upper-triangular W, per precision
-	// register-FFT column pass variant per precision (kColRegSmem / kColTma):
-	// -1 until tuned at the first time step of that precision
-	int col_variant[2] = {-1, -1};
 	int col_forced = -1;  // itp2d_set_column_variant
 	double* lstat = nullptr;     // device: max |E|, |E|_F^2, bad diagonal
 	double* hlstat = nullptr;    // pinned copy
@@ -507,44 +502,8 @@ void col_pass(itp2d_ctx* c, const LinePlan& lp, void* data, const void* mul2d, c
 	a.sx = c->sx; a.sy = c->sy; a.G = c->G;
 	a.cols_per_tile = col_tile_cols(line_len(lp), sizeof(c2<R>), c->sx);
 	a.lp = lp;
-	const int v = c->col_forced >= 0 ? c->col_forced : c->col_variant[c->precision];
-	a.variant = v >= 0 ? v : kColRegSmem;
-	a.err = c->dflag;
 	launch_col_pass<R>(a, c->k, nullptr, c->stream);
 	c->launches++;
-}
-
-// Times the column pass variants on the spare state buffer (its contents are
-// scratch between calls) with the first member's kinetic table, on up to 1024
-// states, and keeps the fastest for this precision.
-template <class R>
-int tune_columns(itp2d_ctx* c) {
-	if (c->boundary != ITP2D_PERIODIC || c->members.empty()) return ITP2D_OK;
-	const MemberTables& mt = c->members[0];
-	ColPassArgs a;
-	a.data = c->acc;
-	a.mul2d = c->B == 0 ? mt.kmul : nullptr;
-	a.mul1d = c->B == 0 ? nullptr : mt.ky;
-	a.mode = 0;
-	a.sx = c->sx; a.sy = c->sy; a.G = c->G;
-	const LinePlan& ly = plan(c, 1, 0);
-	a.cols_per_tile = col_tile_cols(line_len(ly), sizeof(c2<R>), c->sx);
-	a.lp = ly;
-	a.err = c->dflag;
-	// up to 1024 states: enough tiles (32 per state at 512 points) for the
-	// occupancy and tail of a full pass
-	const int v = tune_col_pass_reg<R>(a, std::min(c->k, 1024), c->stream);
-	c->col_variant[c->precision] = v >= 0 ? v : kColRegSmem;
-	ITP2D_TRY(cudaGetLastError());
-	ITP2D_TRY(cudaStreamSynchronize(c->stream));
-	// a time-out of the TMA variant during tuning is reported, not hidden
-	ITP2D_TRY(cudaMemcpy(c->hflag, c->dflag, sizeof(int), cudaMemcpyDeviceToHost));
-	if (*c->hflag != ITP2D_OK) {
-		const int f = *c->hflag;
-		ITP2D_TRY(cudaMemset(c->dflag, 0, sizeof(int)));
-		return f;
-	}
-	return ITP2D_OK;
 }
 
 // One SecondOrderSplit member t applied to `src`, result in `dst`, optionally
@@ -627,12 +586,12 @@ int propagate_fused(itp2d_ctx* c) {
 
 // Row / column tile of the energy passes: the register-FFT tile where that
 // path applies, else the shared-memory tile.
-int energy_rows(const LinePlan& lp, int elem, int sy) {
-	const int r = energy_row_tile_reg(lp, sy);
+int energy_rows(const LinePlan& lp, int elem, int sy, int k) {
+	const int r = energy_row_tile_reg(lp, sy, k);
 	return r ? r : row_tile_rows(line_len(lp), elem, sy);
 }
 int energy_cols(const LinePlan& lp, int elem, int sx) {
-	const int c = energy_col_tile_reg(lp, sx);
+	const int c = energy_col_tile_reg(lp, elem);
 	return c ? c : col_tile_cols(line_len(lp), elem, sx);
 }
 
@@ -650,7 +609,7 @@ int energies_impl(itp2d_ctx* c, void* h_out, bool want_sums) {
 		a.src_t = c->acc; a.psi = c->psi; a.tmul = nullptr; a.V = V;
 		a.h_out = h_out; a.sums = want_sums ? c->sums : nullptr; a.Eshift = c->dEshift;
 		a.do_fwd = 0; a.sx = c->sx; a.sy = c->sy; a.G = c->G;
-		a.rows_per_tile = energy_rows(lx, sizeof(c2<R>), c->sy);
+		a.rows_per_tile = energy_rows(lx, sizeof(c2<R>), c->sy, c->k);
 		a.lp = lx;
 		launch_energy_row<R>(a, c->k, nullptr, c->stream);
 		c->launches++;
@@ -681,7 +640,7 @@ int energies_impl(itp2d_ctx* c, void* h_out, bool want_sums) {
 			a.src_t = src; a.psi = src; a.tmul = c->eTx; a.V = V;
 			a.h_out = c->acc; a.sums = nullptr; a.Eshift = nullptr;
 			a.do_fwd = 1; a.sx = c->sx; a.sy = c->sy; a.G = c->G;
-			a.rows_per_tile = energy_rows(lx, sizeof(c2<R>), c->sy);
+			a.rows_per_tile = energy_rows(lx, sizeof(c2<R>), c->sy, c->k);
 			a.lp = lx;
 			launch_energy_row<R>(a, c->k, nullptr, c->stream);
 		}
@@ -916,33 +875,11 @@ int itp2d_set_time_step(itp2d_ctx* c, double eps) {
 	std::lock_guard<std::mutex> g(c->mu);
 	c->eps = eps;
 	c->eps_set = true;
-	const int st = rebuild_tables(c);
-	if (st || c->col_variant[c->precision] >= 0) return st;
-	// one tuning per device, precision and grid for the process: contexts of
-	// the same size (a serving loop, a batch) reuse the choice
-	static std::mutex mu;
-	static std::map<std::tuple<int, int, int, int, int>, int> tuned;
-	int dev = 0;
-	cudaGetDevice(&dev);
-	const auto key = std::make_tuple(dev, c->precision, c->sx, c->sy, c->boundary);
-	{
-		std::lock_guard<std::mutex> lk(mu);
-		const auto it = tuned.find(key);
-		if (it != tuned.end()) {
-			c->col_variant[c->precision] = it->second;
-			return ITP2D_OK;
-		}
-	}
-	const int r = c->precision == ITP2D_FP64 ? tune_columns<double>(c) : tune_columns<float>(c);
-	if (r == ITP2D_OK && c->col_variant[c->precision] >= 0) {
-		std::lock_guard<std::mutex> lk(mu);
-		tuned[key] = c->col_variant[c->precision];
-	}
-	return r;
+	return rebuild_tables(c);
 }
 
 int itp2d_set_column_variant(itp2d_ctx* c, int variant) {
-	if (!c || variant < -1 || variant >= kColVariants) return ITP2D_E_INVALID;
+	if (!c || variant < -1 || variant > 1) return ITP2D_E_INVALID;
 	std::lock_guard<std::mutex> g(c->mu);
 	c->col_forced = variant;
 	return ITP2D_OK;
@@ -951,8 +888,7 @@ int itp2d_set_column_variant(itp2d_ctx* c, int variant) {
 int itp2d_column_variant(itp2d_ctx* c) {
 	if (!c) return -1;
 	std::lock_guard<std::mutex> g(c->mu);
-	const int v = c->col_forced >= 0 ? c->col_forced : c->col_variant[c->precision];
-	return v >= 0 ? v : kColRegSmem;
+	return c->col_forced >= 0 ? c->col_forced : 0;
 }
 
 int itp2d_upload_states(itp2d_ctx* c, const double* h) {
@@ -1019,15 +955,8 @@ int itp2d_energies(itp2d_ctx* c, double* E, double* sigma, double* sres, double*
 		// the current energies are the shift of the next residual evaluation
 		ITP2D_TRY(cudaMemcpyAsync(c->dEshift, c->dE, (size_t)c->k * sizeof(double), cudaMemcpyDeviceToDevice,
 				c->stream));
-		// status of the bounded waits of the passes since the last check
-		ITP2D_TRY(cudaMemcpyAsync(c->hflag, c->dflag, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
 	}
 	ITP2D_TRY(cudaStreamSynchronize(c->stream));
-	if (*c->hflag != ITP2D_OK) {
-		const int f = *c->hflag;
-		ITP2D_TRY(cudaMemset(c->dflag, 0, sizeof(int)));
-		return f;
-	}
 	const int k = c->k;
 	std::memcpy(E, c->hbuf, k * sizeof(double));
 	std::memcpy(sigma, c->hbuf + k, k * sizeof(double));

@@ -40,13 +40,7 @@ struct ColPassArgs {
 	long long G;
 	int cols_per_tile;
 	LinePlan lp;
-	// register-FFT column pass variant (rfft.cu): kColRegSmem stages tiles
-	// through registers, kColTma by TMA (tune_col_pass_reg picks one per size)
-	int variant = 0;
-	int* err = nullptr;  // device status word for the TMA variant's bounded waits
 };
-
-enum { kColRegSmem = 0, kColTma = 1, kColVariants = 2 };
 
 // Energy pass over rows, producing h = H psi pieces and per-tile sums.
 //   src_t: array whose rows are transformed (psi or a partially transformed
@@ -120,20 +114,25 @@ template <class R> void launch_dm_row_pass(const DmRowArgs& a, int k, cudaStream
 int dm_row_tile_rows(int sx, int elem_bytes, int sy);
 
 template <class R> void launch_row_pass(const RowPassArgs& a, int k, const void* tw, cudaStream_t s);
-// Register-FFT passes (rfft.cu) for periodic lines of 32..1024 points (powers
-// of two); return false, launching nothing, for other lines.
+// Register-FFT passes (lines.cuh) for periodic lines of the lengths of
+// lines::for_length; return false, launching nothing, for other lines.
 template <class R> bool launch_row_pass_reg(const RowPassArgs& a, int k, cudaStream_t s);
 template <class R> bool launch_col_pass_reg(const ColPassArgs& a, int k, cudaStream_t s);
-// Times the register-FFT column pass variants of `a` (its data pointer is a
-// scratch state array of k states, overwritten) and returns the fastest, or
-// -1 if the size has no register path.
-template <class R> int tune_col_pass_reg(ColPassArgs a, int k, cudaStream_t s);
-// Register-FFT energy passes; they run when the tile size equals
-// energy_row_tile_reg / energy_col_tile_reg (non-zero for supported lines).
-int energy_row_tile_reg(const LinePlan& lp, int sy);
-int energy_col_tile_reg(const LinePlan& lp, int sx);
+// Register-FFT energy passes; their tile sizes are energy_row_tile_reg rows
+// (of k states' sy rows) and energy_col_tile_reg columns, 0 for lines they do
+// not take.
+int energy_row_tile_reg(const LinePlan& lp, int sy, int k);
+int energy_col_tile_reg(const LinePlan& lp, int elem_bytes);
 template <class R> bool launch_energy_row_reg(const EnergyRowArgs& a, int k, cudaStream_t s);
 template <class R> bool launch_energy_col_reg(const EnergyColArgs& a, int k, cudaStream_t s);
+template <> bool launch_row_pass_reg<double>(const RowPassArgs&, int, cudaStream_t);
+template <> bool launch_row_pass_reg<float>(const RowPassArgs&, int, cudaStream_t);
+template <> bool launch_col_pass_reg<double>(const ColPassArgs&, int, cudaStream_t);
+template <> bool launch_col_pass_reg<float>(const ColPassArgs&, int, cudaStream_t);
+template <> bool launch_energy_row_reg<double>(const EnergyRowArgs&, int, cudaStream_t);
+template <> bool launch_energy_row_reg<float>(const EnergyRowArgs&, int, cudaStream_t);
+template <> bool launch_energy_col_reg<double>(const EnergyColArgs&, int, cudaStream_t);
+template <> bool launch_energy_col_reg<float>(const EnergyColArgs&, int, cudaStream_t);
 template <class R> void launch_col_pass(const ColPassArgs& a, int k, const void* tw, cudaStream_t s);
 template <class R> void launch_energy_row(const EnergyRowArgs& a, int k, const void* tw, cudaStream_t s);
 template <class R> void launch_energy_col(const EnergyColArgs& a, int k, const void* tw, cudaStream_t s);
