@@ -68,15 +68,16 @@ __global__ void __launch_bounds__(256) overlap_kernel(const T* __restrict__ psi,
 			accr[a][b][0] = accr[a][b][1] = 0.0;
 			acci[a][b][0] = acci[a][b][1] = 0.0;
 		}
-	// loader mapping: row = tid / 4, 4 consecutive complex at seg*4, for A and B
-	const int lrow = tid >> 2, lseg = (tid & 3) * 4;
+	// loader: 16 consecutive lanes copy the 16 points of one row (whole 256-byte
+	// segments of global memory and of the stage)
 	auto fetch = [&](T* st, long long g) {
-		const int ia = i0 + lrow, jb = j0 + lrow;
 #pragma unroll
-		for (int q = 0; q < 4; q++) {
-			const long long gg = g + lseg + q;
-			T* da = st + lrow * kPad + lseg + q;
-			T* db = st + (kBM + lrow) * kPad + lseg + q;
+		for (int q = 0; q < kBM * kBK / 256; q++) {
+			const int e = tid + q * 256, row = e / kBK, p = e % kBK;
+			const int ia = i0 + row, jb = j0 + row;
+			const long long gg = g + p;
+			T* da = st + row * kPad + p;
+			T* db = st + (kBM + row) * kPad + p;
 			if (gg < g1 && ia < k) cp_async_elem<T>(da, psi + (long long)ia * G + gg);
 			else *da = T{0, 0};
 			if (gg < g1 && jb < k) cp_async_elem<T>(db, psib + (long long)jb * G + gg);
@@ -139,18 +140,32 @@ __global__ void __launch_bounds__(256) overlap_kernel(const T* __restrict__ psi,
 }
 
 // Sum the splits (fixed order), scale, and build the Hermitian matrix from the
-// upper triangle. One thread per (i, j) with i <= j of the full matrix.
-__global__ void overlap_finish_kernel(const double2* __restrict__ part, int k, int nsplit, double dx2,
-		double2* __restrict__ S) {
-	const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-	if (idx >= (long long)k * k) return;
+// upper triangle: 32 elements by 8 groups of splits per CTA (group y sums the
+// splits y, y + 8, ...; the groups are added in order), so that a small matrix
+// with many splits is not one chain of loads per element.
+constexpr int kFinishGroups = 8;
+__global__ void __launch_bounds__(32 * kFinishGroups) overlap_finish_kernel(const double2* __restrict__ part, int k,
+		int nsplit, double dx2, double2* __restrict__ S) {
+	__shared__ double2 red[kFinishGroups][32];
+	const long long kk = (long long)k * k;
+	const long long idx = (long long)blockIdx.x * 32 + threadIdx.x;
 	const int i = (int)(idx / k), j = (int)(idx % k);
-	if (i > j) return;
+	const bool on = idx < kk && i <= j;
 	double sr = 0.0, si = 0.0;
-	for (int s = 0; s < nsplit; s++) {
-		const double2 v = part[(size_t)s * k * k + idx];
-		sr += v.x;
-		si += v.y;
+	if (on) {
+#pragma unroll 4
+		for (int s = threadIdx.y; s < nsplit; s += kFinishGroups) {
+			const double2 v = part[(size_t)s * kk + idx];
+			sr += v.x;
+			si += v.y;
+		}
+	}
+	red[threadIdx.y][threadIdx.x] = make_double2(sr, si);
+	__syncthreads();
+	if (threadIdx.y || !on) return;
+	for (int y = 1; y < kFinishGroups; y++) {
+		sr += red[y][threadIdx.x].x;
+		si += red[y][threadIdx.x].y;
 	}
 	sr *= dx2;
 	si *= dx2;
@@ -310,13 +325,15 @@ int overlap_splits(int k, long long G, int num_sms) {
 	const int nt = overlap_tiles(k);
 	const long long npairs = (long long)nt * (nt + 1) / 2;
 	// two CTAs per SM (80 KB of stages each for FP64 states); splits of at
-	// least 512 grid points, up to enough for two waves (at least 16); the
+	// least 128 grid points (8 steps: fewer would not cover the two latencies at
+	// their ends; 512 left 18 CTAs for 48 states on 96 x 96 and took 105 us,
+	// 37 us now), up to enough for two waves (at least 16); the
 	// first count whose grid fills its last wave to 95 % or more, else the
 	// best-filled one (k = 2000: 528 tile pairs fill 1.78 waves unsplit, 5
 	// splits fill 8.92 waves; a few tile pairs take as many splits as fill
 	// the GPU)
 	const long long slots = 2LL * num_sms;
-	const long long most = std::max(1LL, std::min(G / 512, std::max(16LL, 2 * slots / npairs)));
+	const long long most = std::max(1LL, std::min(G / 128, std::max(16LL, 2 * slots / npairs)));
 	long long best = 1;
 	double best_fill = 0.0;
 	for (long long ns = 1; ns <= most; ns++) {
@@ -346,7 +363,7 @@ void launch_overlap(const T* psi, int k, long long G, const int2* pairs, int npa
 
 void launch_overlap_finish(const double2* part, int k, int nsplit, double dx2, double2* S, cudaStream_t s) {
 	const long long kk = (long long)k * k;
-	overlap_finish_kernel<<<(unsigned)((kk + 255) / 256), 256, 0, s>>>(part, k, nsplit, dx2, S);
+	overlap_finish_kernel<<<(unsigned)((kk + 31) / 32), dim3(32, kFinishGroups), 0, s>>>(part, k, nsplit, dx2, S);
 }
 
 template <class T>
