@@ -462,13 +462,13 @@ struct Geo {
 	static constexpr int ENERGY_COL_BLOCKS = blocks(COL_THREADS, ES == 16 ? 40 : 16);
 };
 
-// Forward twiddles w_N^(b k1) at [k1 * LD + b].
-template <class R, class G, int LD>
+// Forward twiddles w_N^(b k1) at [k1 * LD + b]; tw[ST j] = w_N^j.
+template <class R, class G, int LD, int ST = 1>
 __device__ __forceinline__ void load_tw(c2<R>* xtw, const void* tw) {
 	const c2<R>* g = reinterpret_cast<const c2<R>*>(tw);
 	for (int i = threadIdx.x; i < G::N; i += blockDim.x) {
 		const int k1 = i / G::B, b = i - k1 * G::B;
-		xtw[k1 * LD + b] = g[b * k1];  // b k1 < N
+		xtw[k1 * LD + b] = g[ST * b * k1];  // b k1 < N
 	}
 }
 

@@ -118,6 +118,9 @@ template <class R> void launch_row_pass(const RowPassArgs& a, int k, const void*
 // lines::for_length; return false, launching nothing, for other lines.
 template <class R> bool launch_row_pass_reg(const RowPassArgs& a, int k, cudaStream_t s);
 template <class R> bool launch_col_pass_reg(const ColPassArgs& a, int k, cudaStream_t s);
+// The same for Dirichlet lines (sine transforms, lines_dst.cuh).
+template <class R> bool launch_row_pass_sine(const RowPassArgs& a, int k, cudaStream_t s);
+template <class R> bool launch_col_pass_sine(const ColPassArgs& a, int k, cudaStream_t s);
 // Register-FFT energy passes; their tile sizes are energy_row_tile_reg rows
 // (of k states' sy rows) and energy_col_tile_reg columns, 0 for lines they do
 // not take.
@@ -129,6 +132,10 @@ template <> bool launch_row_pass_reg<double>(const RowPassArgs&, int, cudaStream
 template <> bool launch_row_pass_reg<float>(const RowPassArgs&, int, cudaStream_t);
 template <> bool launch_col_pass_reg<double>(const ColPassArgs&, int, cudaStream_t);
 template <> bool launch_col_pass_reg<float>(const ColPassArgs&, int, cudaStream_t);
+template <> bool launch_row_pass_sine<double>(const RowPassArgs&, int, cudaStream_t);
+template <> bool launch_row_pass_sine<float>(const RowPassArgs&, int, cudaStream_t);
+template <> bool launch_col_pass_sine<double>(const ColPassArgs&, int, cudaStream_t);
+template <> bool launch_col_pass_sine<float>(const ColPassArgs&, int, cudaStream_t);
 template <> bool launch_energy_row_reg<double>(const EnergyRowArgs&, int, cudaStream_t);
 template <> bool launch_energy_row_reg<float>(const EnergyRowArgs&, int, cudaStream_t);
 template <> bool launch_energy_col_reg<double>(const EnergyColArgs&, int, cudaStream_t);

@@ -77,3 +77,43 @@ def test_step_hamiltonian_and_energies_match_oracle(capi, shape, B, precision):
         assert _rel(h, O.Hamiltonian(g, V, O.PERIODIC, B).apply(psi)) < tol
         assert np.max(np.abs(E - mean.real)) < etol * np.max(np.abs(mean))
         assert np.max(np.abs(sigma - sd.real)) < etol * np.max(np.abs(sd))
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+@pytest.mark.parametrize("n", LENGTHS)
+def test_sine_transforms_match_oracle(capi, n, precision):
+    rng = np.random.default_rng(n)
+    prec = capi.FP64 if precision == "fp64" else capi.FP32
+    for sx, sy, kinds in [(n, 7, ("DSTx", "iDSTx")), (21, n, ("DSTy", "iDSTy"))]:
+        psi = rng.standard_normal((3, sy, sx)) + 1j * rng.standard_normal((3, sy, sx))
+        c = capi.Context(sx, sy, 0.1, 3, capi.DIRICHLET, precision=prec)
+        for kind in kinds:
+            c.upload(psi)
+            c.transform(kind)
+            assert _rel(c.download(), O.transform(psi, kind)) < TOL[precision], (sx, sy, kind)
+        c.close()
+
+
+# even and odd factors (item A / 2 exists or not, N / 2 in item 0 or A / 2), both
+# accumulating and in-place members
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+@pytest.mark.parametrize("shape", [(64, 90), (90, 40), (150, 100), (36, 225), (240, 72), (512, 9)])
+def test_dirichlet_step_matches_oracle(capi, shape, precision):
+    sx, sy = shape
+    g = O.Grid(sx, sy, 0.15)
+    V = O.harmonic(g)
+    for k, m in [(1, 1), (4, 3)]:
+        psi = O.gaussian_states(g, k, 3)
+        c = capi.Context(sx, sy, g.dx, k, capi.DIRICHLET, 0.0, m, capi.FP64 if precision == "fp64" else capi.FP32)
+        c.set_potential(V)
+        c.set_time_step(0.05)
+        c.upload(psi)
+        c.propagate()
+        step = c.download()
+        c.upload(psi)
+        c.apply_hamiltonian()
+        h = c.download()
+        c.close()
+        tol = 1e-12 if precision == "fp64" else 2e-5
+        assert _rel(step, O.MultiProductSplit(g, V, O.DIRICHLET, 0.0, m, 0.05).apply(psi)) < tol
+        assert _rel(h, O.Hamiltonian(g, V, O.DIRICHLET, 0.0).apply(psi)) < tol
