@@ -133,7 +133,7 @@ cudaError_t launch_ritz(double2* H, int k, JacobiWork& w, double2* W, EigStatus*
 // gives up sets *err to ITP2D_E_TIMEOUT. upper: W upper triangular. The
 // overlap writes nsplit (oz_overlap_splits, at most max_splits) partial
 // blocks into part and sums them into S (launch_overlap_finish).
-// oz_launches() kernels per call of either.
+// oz_overlap_launches() and oz_rotate_launches() kernels per call.
 bool oz_supported(int k, long long G);
 size_t oz_w_bytes(int k);
 size_t oz_scratch_bytes(int k, long long G);
@@ -143,7 +143,8 @@ void launch_rotate_oz(const double2* W, const double2* psi, int k, long long G, 
 int oz_overlap_splits(int k, long long G, int num_sms, int max_splits);
 void launch_overlap_oz(const double2* psi, int k, long long G, int nsplit, unsigned char* scratch, int* ebuf,
 		double2* part, double dx2, double2* S, int* err, cudaStream_t s);
-int oz_launches();
+int oz_overlap_launches();
+int oz_rotate_launches();
 
 // Second-order Lowdin orthonormalisation (lowdin.cu): D = diag(S)^{-1/2},
 // E = D S D - I (row-major) and conj(E), stats = {max |E_ij|, sum |E_ij|^2,

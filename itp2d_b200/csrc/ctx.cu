@@ -1031,7 +1031,7 @@ void launch_overlap_any(itp2d_ctx* c, bool tc, bool int8 = true) {
 	if (int8 && !tc && c->precision == ITP2D_FP64 && oz_ready(c)) {
 		launch_overlap_oz((const double2*)c->psi, c->k, c->G, c->oz_nsplit, c->oz_scratch, c->oz_e, c->part,
 				c->dx * c->dx, c->S, c->dflag, c->stream);
-		c->launches += oz_launches();
+		c->launches += oz_overlap_launches();
 		c->oz_calls++;
 		return;
 	}
@@ -1186,7 +1186,7 @@ static int rotate_states(itp2d_ctx* c, bool tc, bool upper = false) {
 					(double2*)c->acc, c->dflag, c->stream, upper);
 		else if (f64) launch_rotate(c->W, (const double2*)c->psi, c->k, c->G, (double2*)c->acc, c->stream, upper);
 		else launch_rotate(c->W, (const float2*)c->psi, c->k, c->G, (float2*)c->acc, c->stream, upper);
-		c->launches += tc ? 2 : (oz ? oz_launches() : 1);
+		c->launches += tc ? 2 : (oz ? oz_rotate_launches() : 1);
 	}
 	if (oz) c->oz_calls++;
 	const bool flagged = tc || oz;
@@ -1366,7 +1366,7 @@ int itp2d_orthonormalize(itp2d_ctx* c, int algo, int* bad_index, double* bad_val
 					(double2*)c->acc, c->dflag, c->stream, false);
 		else if (f64) launch_rotate(c->W, (const double2*)c->psi, c->k, c->G, (double2*)c->acc, c->stream);
 		else launch_rotate(c->W, (const float2*)c->psi, c->k, c->G, (float2*)c->acc, c->stream);
-		c->launches += tc ? 2 : (oz ? oz_launches() : 1);
+		c->launches += tc ? 2 : (oz ? oz_rotate_launches() : 1);
 	}
 	if (oz) c->oz_calls++;
 	const bool flagged = tc || oz;

@@ -26,9 +26,9 @@
 //   * pre-split (the default): split_psi_rows_kernel / split_psi_cols_kernel
 //     write the planes of the states once per contraction, in the MMA block
 //     layout; overlap_tc2_kernel / rotate_tc2_kernel then run their K loop in
-//     one thread: a cp.async.bulk of each 24 KB block into a ring of four
-//     slots (full mbarrier), the 24 MMAs, tcgen05.commit to the slot's empty
-//     mbarrier, and the refill of the previous step's slot;
+//     two threads: one copies each 24 KB block (cp.async.bulk) into a ring of
+//     four slots (full mbarrier), the other issues the 24 MMAs of a step and
+//     tcgen05.commits them to the slot's empty mbarrier;
 //   * staged (ITP2D_CONTRACT_TC_STAGED): overlap_tc_kernel / rotate_tc_kernel
 //     split inside the CTA. Per step:
 //   * cp.async fetches the FP32 operand tiles of step s + 2 into a ring of
@@ -431,61 +431,63 @@ constexpr int kRing = 4;                      // slots of (A, B) block pairs
 constexpr int kSlotBytes = 2 * kOperandBytes;  // 48 KB
 static_assert(kRing * kSlotBytes <= kBufBytes, "pre-split ring");
 
-// The K loop over pre-split blocks, run by thread 0 alone: block pair s is
-// copied into slot s mod kRing (full[slot] completes when it has landed),
-// its MMAs are issued and committed to empty[slot]; after the MMAs of step s
-// are issued, the slot of step s - 1 is refilled with step s - 1 + kRing once
-// those MMAs have finished reading it. src_a(s) / src_b(s) give the global
-// blocks (src_b null: B reads A's planes). Returns with every MMA complete or
-// with sh.abort set (copies and MMAs in flight drained, bounded).
+// The K loop over pre-split blocks (all threads call it). Thread 32 copies block
+// pair s into slot s mod kRing (full[slot] completes when it has landed), for s >=
+// kRing once the MMAs of step s - kRing have read the slot; thread 0 issues the
+// MMAs of step s and commits them to empty[slot]. Two threads, because issuing
+// blocks at the tensor pipe's rate: with the copies and their waits in the same
+// thread the pipe idled a third of the time between steps. src_a(s) / src_b(s)
+// give the global blocks (src_b null: B reads A's planes). Returns, after a block
+// barrier, with every MMA complete or with sh.abort set (copies and MMAs in
+// flight drained, bounded).
 template <class SrcA, class SrcB>
 __device__ void run_bulk_pipeline(TcShared& sh, unsigned long long* full, unsigned long long* empty, int nsteps,
 		bool conjA, SrcA src_a, SrcB src_b, int* err) {
-	if (threadIdx.x != 0 || nsteps <= 0) return;
+	__shared__ int s_copied;
 	unsigned char* const base = sh.buf;
-	auto copy = [&](int st) {
-		const int slot = st % kRing;
-		unsigned char* dst = base + slot * kSlotBytes;
-		const unsigned char* b = src_b(st);
-		const uint32_t fb = smem_u32(&full[slot]);
-		mbar_expect_tx(fb, b ? 2 * kOperandBytes : kOperandBytes);
-		bulk_copy(smem_u32(dst), src_a(st), kOperandBytes, fb);
-		if (b) bulk_copy(smem_u32(dst + kOperandBytes), b, kOperandBytes, fb);
+	int issued = 0;  // thread 0: steps whose MMAs were issued
+	auto give_up = [&]() {
+		sh.abort = 1;
+		atomicExch(err, ITP2D_E_TIMEOUT);
 	};
-	int copied = 0, issued = 0;  // steps copied / whose MMAs were issued
-	for (; copied < nsteps && copied < kRing; copied++) copy(copied);
-	bool ok = true;
-	for (int st = 0; st < nsteps; st++) {
-		const int slot = st % kRing;
-		if (!mbar_wait(smem_u32(&full[slot]), (uint32_t)((st / kRing) & 1))) {
-			ok = false;
-			break;
-		}
-		tc_fence_after();
-		const uint32_t a = smem_u32(base + slot * kSlotBytes);
-		issue_step(sh.tmem_base, a, src_b(st) ? a + kOperandBytes : a, conjA, st == 0);
-		umma_commit(smem_u32(&empty[slot]));
-		issued = st + 1;
-		if (st >= 1 && copied < nsteps) {
-			const int ps = (st - 1) % kRing;
-			if (!mbar_wait(smem_u32(&empty[ps]), (uint32_t)(((st - 1) / kRing) & 1))) {
-				ok = false;
+	if (threadIdx.x == 32) {
+		int st = 0;
+		for (; st < nsteps; st++) {
+			const int slot = st % kRing;
+			if (st >= kRing && !mbar_wait(smem_u32(&empty[slot]), (uint32_t)((st / kRing - 1) & 1))) {
+				give_up();
 				break;
 			}
-			copy(copied++);
+			unsigned char* dst = base + slot * kSlotBytes;
+			const unsigned char* b = src_b(st);
+			const uint32_t fb = smem_u32(&full[slot]);
+			mbar_expect_tx(fb, b ? 2 * kOperandBytes : kOperandBytes);
+			bulk_copy(smem_u32(dst), src_a(st), kOperandBytes, fb);
+			if (b) bulk_copy(smem_u32(dst + kOperandBytes), b, kOperandBytes, fb);
 		}
+		s_copied = st;
 	}
-	if (!ok) {
-		sh.abort = 1;
-		atomicExch(err, ITP2D_E_TIMEOUT);
-		// copies not yet waited for land before the CTA leaves
-		for (int st = issued; st < copied; st++) mbar_wait(smem_u32(&full[st % kRing]), (uint32_t)((st / kRing) & 1));
+	if (threadIdx.x == 0) {
+		for (int st = 0; st < nsteps; st++) {
+			const int slot = st % kRing;
+			if (!mbar_wait(smem_u32(&full[slot]), (uint32_t)((st / kRing) & 1))) {
+				give_up();
+				break;
+			}
+			tc_fence_after();
+			const uint32_t a = smem_u32(base + slot * kSlotBytes);
+			issue_step(sh.tmem_base, a, src_b(st) ? a + kOperandBytes : a, conjA, st == 0);
+			umma_commit(smem_u32(&empty[slot]));
+			issued = st + 1;
+		}
+		// the last commit covers every MMA issued before it
+		if (issued > 0 && !mbar_wait(smem_u32(&empty[(issued - 1) % kRing]), (uint32_t)(((issued - 1) / kRing) & 1)))
+			give_up();
 	}
-	// the last commit covers every MMA issued before it
-	if (issued > 0 && !mbar_wait(smem_u32(&empty[(issued - 1) % kRing]), (uint32_t)(((issued - 1) / kRing) & 1))) {
-		sh.abort = 1;
-		atomicExch(err, ITP2D_E_TIMEOUT);
-	}
+	__syncthreads();
+	// copies not waited for land before the CTA leaves
+	if (sh.abort && threadIdx.x == 0)
+		for (int st = issued; st < s_copied; st++) mbar_wait(smem_u32(&full[st % kRing]), (uint32_t)((st / kRing) & 1));
 }
 
 __device__ void init_ring(unsigned long long* full, unsigned long long* empty) {

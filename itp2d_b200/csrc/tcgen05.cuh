@@ -76,7 +76,7 @@ __device__ __forceinline__ unsigned long long global_ns() {
 // Bounded wait for the phase with the given parity: false once kWaitNs of
 // wall time (or kSpinLimit polls) passed without the phase completing.
 __device__ __forceinline__ bool mbar_wait(uint32_t mbar, uint32_t parity) {
-	const unsigned long long t0 = global_ns();
+	unsigned long long t0 = 0;  // set once the wait turns out to be a longer one
 	for (long long i = 0; i < kSpinLimit; i++) {
 		uint32_t done;
 		asm volatile(
@@ -87,6 +87,7 @@ __device__ __forceinline__ bool mbar_wait(uint32_t mbar, uint32_t parity) {
 				: "r"(mbar), "r"(parity)
 				: "memory");
 		if (done) return true;
+		if (i == 16) t0 = global_ns();
 		if (i > 64) {
 			__nanosleep(64);
 			if ((i & 255) == 0 && global_ns() - t0 > kWaitNs) return false;
