@@ -48,18 +48,30 @@ __global__ void chol_identity_kernel(double2* X, int k) {
 		X[i] = make_double2(i / k == i % k ? 1.0 : 0.0, 0.0);
 }
 
-// Step 1: L_jj and L_jj^{-1} of the diagonal block at (j, j); 1024 threads.
+// Step 1: L_jj and L_jj^{-1} of the diagonal block at (j, j); 1024 threads,
+// thread (r, c) holding element (r, c) of the block and of its inverse in
+// registers. The inverse is built along with the factor (forward substitution
+// of the identity: row p of X is final once it is divided by the pivot), two
+// barriers per pivot; the thread of the next pivot prepares its reciprocal
+// square root right after its update. Latency-bound: a chain of 32 pivots
+// (39 us with the inverse substituted afterwards by one thread per column,
+// 20 us now).
 __global__ void __launch_bounds__(1024) chol_diag_kernel(double2* A, int k, int j, double2* Linv, EigStatus* st) {
-	__shared__ double2 L[NB][NB + 1];
-	__shared__ double2 M[NB][NB + 1];
+	__shared__ double2 lcol[NB], xrow[NB];  // column p of L, row p of X
+	__shared__ double s_pivot[2], s_inv[2];
 	if (st->status != 0) return;
 	const int nb = min(NB, k - j);
 	const int r = threadIdx.x / NB, c = threadIdx.x % NB;
-	L[r][c] = (r < nb && c < nb && c <= r) ? A[(long long)(j + r) * k + j + c] : make_double2(0.0, 0.0);
-	M[r][c] = make_double2(0.0, 0.0);
+	const bool in = r < nb && c <= r;
+	double2 l = in ? A[(long long)(j + r) * k + j + c] : make_double2(0.0, 0.0);
+	double2 x = make_double2(r == c ? 1.0 : 0.0, 0.0);
+	if (threadIdx.x == 0) {
+		s_pivot[0] = l.x;
+		s_inv[0] = rsqrt(l.x);
+	}
+	__syncthreads();
 	for (int p = 0; p < nb; p++) {
-		__syncthreads();
-		const double pivot = L[p][p].x;
+		const double pivot = s_pivot[p & 1], inv = s_inv[p & 1];
 		if (!(pivot > 0.0) || !isfinite(pivot)) {
 			if (threadIdx.x == 0) {
 				st->status = ITP2D_E_NONPOSITIVE_EIGENVALUE;
@@ -68,29 +80,31 @@ __global__ void __launch_bounds__(1024) chol_diag_kernel(double2* A, int k, int 
 			}
 			return;  // every thread read the same pivot: the whole CTA leaves here
 		}
-		const double d = sqrt(pivot);
-		__syncthreads();
-		if (c == p && r >= p && r < nb) {
-			const double2 v = L[r][p];
-			L[r][p] = r == p ? make_double2(d, 0.0) : make_double2(v.x / d, v.y / d);
+		if (c == p && r >= p) {
+			l = r == p ? make_double2(pivot * inv, 0.0) : make_double2(l.x * inv, l.y * inv);
+			lcol[r] = l;
+		}
+		if (r == p && c <= p) {
+			x = make_double2(x.x * inv, x.y * inv);
+			xrow[c] = x;
 		}
 		__syncthreads();
-		if (c > p && r >= c && r < nb) L[r][c] = csub(L[r][c], cmulc(L[r][p], L[c][p]));
-	}
-	__syncthreads();
-	if (r < nb && c <= r) A[(long long)(j + r) * k + j + c] = L[r][c];
-	// L^{-1} column by column (one thread per column, forward substitution)
-	if (threadIdx.x < nb) {
-		const int col = threadIdx.x;
-		for (int row = col; row < nb; row++) {
-			double2 s = make_double2(row == col ? 1.0 : 0.0, 0.0);
-			for (int m = col; m < row; m++) s = csub(s, cmul(L[row][m], M[m][col]));
-			const double inv = 1.0 / L[row][row].x;
-			M[row][col] = make_double2(s.x * inv, s.y * inv);
+		if (r > p && r < nb) {
+			const double2 lr = lcol[r];
+			if (c > p && c <= r) {
+				l = csub(l, cmulc(lr, lcol[c]));
+				if (r == p + 1) {  // c == r: the next pivot
+					s_pivot[r & 1] = l.x;
+					s_inv[r & 1] = rsqrt(l.x);
+				}
+			}
+			if (c <= p) x = csub(x, cmul(lr, xrow[c]));
 		}
+		__syncthreads();
 	}
-	__syncthreads();
-	Linv[r * NB + c] = M[r][c];  // zero above the diagonal and beyond nb
+	if (in) A[(long long)(j + r) * k + j + c] = l;
+	// zero above the diagonal and beyond nb
+	Linv[r * NB + c] = in ? x : make_double2(0.0, 0.0);
 }
 
 // Step 2: blocks [0, nrb) turn 32 rows of the panel below the diagonal block
@@ -102,27 +116,45 @@ __global__ void __launch_bounds__(256) chol_panel_kernel(double2* A, double2* X,
 	__shared__ double2 T[NB][NB + 1];
 	if (st->status != 0) return;
 	const int nb = min(NB, k - j), r0 = j + nb;
-	for (int i = threadIdx.x; i < NB * NB; i += blockDim.x) Li[i / NB][i % NB] = Linv[i];
+	constexpr int NE = NB * NB / 256;  // outputs per thread: rows rr, rr + 8, ...
 	if ((int)blockIdx.x < nrb) {
 		const int row0 = r0 + NB * blockIdx.x;
-		for (int i = threadIdx.x; i < NB * NB; i += blockDim.x) {
-			const int rr = i / NB, p = i % NB, row = row0 + rr;
-			T[rr][p] = (row < k && p < nb) ? A[(long long)row * k + j + p] : make_double2(0.0, 0.0);
+		const int rr = threadIdx.x / NB, q = threadIdx.x % NB;
+		double2 lv[NE], tv[NE];
+#pragma unroll
+		for (int e = 0; e < NE; e++) {
+			const int row = row0 + rr + 8 * e;
+			lv[e] = __ldcg(Linv + threadIdx.x + 256 * e);
+			tv[e] = (row < k && q < nb) ? __ldcg(A + (long long)row * k + j + q) : make_double2(0.0, 0.0);
+		}
+#pragma unroll
+		for (int e = 0; e < NE; e++) {
+			Li[rr + 8 * e][q] = lv[e];
+			T[rr + 8 * e][q] = tv[e];
 		}
 		__syncthreads();
-		for (int i = threadIdx.x; i < NB * NB; i += blockDim.x) {
-			const int rr = i / NB, q = i % NB, row = row0 + rr;
-			if (row >= k || q >= nb) continue;
-			double2 s = make_double2(0.0, 0.0);
-			for (int p = 0; p <= q; p++) {
-				const double2 a = T[rr][p], l = Li[q][p];
-				s.x += a.x * l.x + a.y * l.y;  // a * conj(l)
-				s.y += a.y * l.x - a.x * l.y;
+		// L^{-1} is zero above its diagonal: the sums run over the whole row
+		double2 s[NE];
+#pragma unroll
+		for (int e = 0; e < NE; e++) s[e] = make_double2(0.0, 0.0);
+#pragma unroll 8
+		for (int p = 0; p < NB; p++) {
+			const double2 l = Li[q][p];
+#pragma unroll
+			for (int e = 0; e < NE; e++) {
+				const double2 a = T[rr + 8 * e][p];
+				s[e].x += a.x * l.x + a.y * l.y;  // a * conj(l)
+				s[e].y += a.y * l.x - a.x * l.y;
 			}
-			A[(long long)row * k + j + q] = s;
+		}
+#pragma unroll
+		for (int e = 0; e < NE; e++) {
+			const int row = row0 + rr + 8 * e;
+			if (row < k && q < nb) A[(long long)row * k + j + q] = s[e];
 		}
 		return;
 	}
+	for (int i = threadIdx.x; i < NB * NB; i += blockDim.x) Li[i / NB][i % NB] = Linv[i];
 	const int c0 = NB * (blockIdx.x - nrb);
 	if (c0 >= j) {
 		// the panel's own columns: X_j = L_jj^{-1} there (identity before)
@@ -132,29 +164,37 @@ __global__ void __launch_bounds__(256) chol_panel_kernel(double2* A, double2* X,
 		}
 		return;
 	}
-	for (int i = threadIdx.x; i < NB * NB; i += blockDim.x) {
-		const int q = i / NB, cc = i % NB;
-		T[q][cc] = q < nb ? X[(long long)(j + q) * k + c0 + cc] : make_double2(0.0, 0.0);
-	}
+	const int q0 = threadIdx.x / NB, cc = threadIdx.x % NB;
+	double2 tv[NE];
+#pragma unroll
+	for (int e = 0; e < NE; e++)
+		tv[e] = q0 + 8 * e < nb ? __ldcg(X + (long long)(j + q0 + 8 * e) * k + c0 + cc) : make_double2(0.0, 0.0);
+#pragma unroll
+	for (int e = 0; e < NE; e++) T[q0 + 8 * e][cc] = tv[e];
 	__syncthreads();
-	for (int i = threadIdx.x; i < NB * NB; i += blockDim.x) {
-		const int q = i / NB, cc = i % NB;
-		if (q >= nb) continue;
-		double2 s = make_double2(0.0, 0.0);
-		for (int p = 0; p <= q; p++) {
-			const double2 l = Li[q][p], x = T[p][cc];
-			s.x += l.x * x.x - l.y * x.y;
-			s.y += l.x * x.y + l.y * x.x;
+	double2 s[NE];
+#pragma unroll
+	for (int e = 0; e < NE; e++) s[e] = make_double2(0.0, 0.0);
+#pragma unroll 8
+	for (int p = 0; p < NB; p++) {
+		const double2 x = T[p][cc];
+#pragma unroll
+		for (int e = 0; e < NE; e++) {
+			const double2 l = Li[q0 + 8 * e][p];
+			s[e].x += l.x * x.x - l.y * x.y;
+			s[e].y += l.x * x.y + l.y * x.x;
 		}
-		X[(long long)(j + q) * k + c0 + cc] = s;
 	}
+#pragma unroll
+	for (int e = 0; e < NE; e++)
+		if (q0 + 8 * e < nb) X[(long long)(j + q0 + 8 * e) * k + c0 + cc] = s[e];
 }
 
 // Step 3: rows [r0, k) of the trailing part. Column tiles [0, ncx) cover X's
 // columns [0, r0) (X_2 -= L_21 X_j); the rest cover A's columns [r0, k)
 // aligned with the row tiles (A_22 -= L_21 L_21^H, lower triangle only).
 // 256 threads, 4 x 4 outputs each.
-__global__ void __launch_bounds__(256) chol_update_kernel(double2* A, double2* X, int k, int j, int ncx,
+__global__ void __launch_bounds__(256, 2) chol_update_kernel(double2* A, double2* X, int k, int j, int ncx,
 		const EigStatus* st) {
 	extern __shared__ __align__(16) unsigned char smem_raw[];
 	double2(*Lt)[NB + 1] = reinterpret_cast<double2(*)[NB + 1]>(smem_raw);             // [TU][NB + 1]
@@ -167,21 +207,27 @@ __global__ void __launch_bounds__(256) chol_update_kernel(double2* A, double2* X
 	const int row0 = r0 + TU * rt;
 	const int col0 = xpart ? TU * ct : r0 + TU * (ct - ncx);
 	const int col_end = xpart ? r0 : k;
-	for (int i = threadIdx.x; i < TU * NB; i += blockDim.x) {
-		const int rr = i / NB, q = i % NB, row = row0 + rr;
-		Lt[rr][q] = (row < k && q < nb) ? A[(long long)row * k + j + q] : make_double2(0.0, 0.0);
-	}
-	for (int i = threadIdx.x; i < TU * NB; i += blockDim.x) {
-		const int q = i / TU, cc = i % TU, col = col0 + cc;
-		double2 b = make_double2(0.0, 0.0);
-		if (q < nb && col < col_end) {
-			if (xpart) b = X[(long long)(j + q) * k + col];
-			else {
-				const double2 l = A[(long long)col * k + j + q];
-				b = make_double2(l.x, -l.y);
-			}
+	// every global load of the tile at once, then the shared-memory stores
+	constexpr int NL = TU * NB / 256;
+	double2 lv[NL], bv[NL];
+#pragma unroll
+	for (int e = 0; e < NL; e++) {
+		const int i = threadIdx.x + 256 * e, rr = i / NB, q = i % NB, row = row0 + rr;
+		lv[e] = (row < k && q < nb) ? __ldcg(A + (long long)row * k + j + q) : make_double2(0.0, 0.0);
+		if (xpart) {
+			const int qq = i / TU, col = col0 + i % TU;
+			bv[e] = (qq < nb && col < col_end) ? __ldcg(X + (long long)(j + qq) * k + col) : make_double2(0.0, 0.0);
+		} else {
+			const int col = col0 + rr;
+			bv[e] = (q < nb && col < col_end) ? __ldcg(A + (long long)col * k + j + q) : make_double2(0.0, 0.0);
 		}
-		Bt[q][cc] = b;
+	}
+#pragma unroll
+	for (int e = 0; e < NL; e++) {
+		const int i = threadIdx.x + 256 * e, rr = i / NB, q = i % NB;
+		Lt[rr][q] = lv[e];
+		if (xpart) Bt[i / TU][i % TU] = bv[e];
+		else Bt[q][rr] = make_double2(bv[e].x, -bv[e].y);
 	}
 	__syncthreads();
 	const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;
@@ -205,17 +251,26 @@ __global__ void __launch_bounds__(256) chol_update_kernel(double2* A, double2* X
 			}
 	}
 	double2* out = xpart ? X : A;
+	// the old values of two rows of outputs at once (the compiler cannot move a
+	// load above an earlier output's store)
 #pragma unroll
-	for (int a = 0; a < 4; a++) {
-		const int row = row0 + ty + 16 * a;
-		if (row >= k) continue;
+	for (int a0 = 0; a0 < 4; a0 += 2) {
+		double2 old[2][4];
 #pragma unroll
-		for (int b = 0; b < 4; b++) {
-			const int col = col0 + tx + 16 * b;
-			if (col >= col_end || (!xpart && col > row)) continue;
-			double2* o = out + (long long)row * k + col;
-			*o = csub(*o, acc[a][b]);
-		}
+		for (int a = 0; a < 2; a++)
+#pragma unroll
+			for (int b = 0; b < 4; b++) {
+				const int row = row0 + ty + 16 * (a0 + a), col = col0 + tx + 16 * b;
+				if (row < k && col < col_end && (xpart || col <= row)) old[a][b] = __ldcg(out + (long long)row * k + col);
+			}
+#pragma unroll
+		for (int a = 0; a < 2; a++)
+#pragma unroll
+			for (int b = 0; b < 4; b++) {
+				const int row = row0 + ty + 16 * (a0 + a), col = col0 + tx + 16 * b;
+				if (row < k && col < col_end && (xpart || col <= row))
+					out[(long long)row * k + col] = csub(old[a][b], acc[a0 + a][b]);
+			}
 	}
 }
 
