@@ -18,7 +18,7 @@ OBJ = os.path.join(HERE, "_build")
 LIB = os.path.join(HERE, "libitp2d_b200.so")
 
 SOURCES = ["split.cu", "contract.cu", "jacobi.cu", "ctx.cu", "probe.cu", "noalloc.cu", "bjacobi.cu", "tc.cu", "lines_row_f64.cu", "lines_row_f32.cu", "lines_col_f64.cu", "lines_col_f32.cu", "lines_energy_f64.cu",
-           "lines_energy_f32.cu", "lines_dst_f64.cu", "lines_dst_f32.cu", "bjacobi32.cu", "potential.cu", "lowdin.cu", "batch.cu", "cholesky.cu", "oz.cu"]
+           "lines_energy_f32.cu", "lines_dst_f64.cu", "lines_dst_f32.cu", "lines_small_f64.cu", "lines_small_f32.cu", "bjacobi32.cu", "potential.cu", "lowdin.cu", "batch.cu", "cholesky.cu", "oz.cu"]
 HOST_SOURCES = [os.path.join("host", "itp2d_host.cpp"), os.path.join("host", "itp2d_serve.cpp"),
                 os.path.join("host", "itp2d_datafile.cpp")]
 CXX_FLAGS = ["-O2", "-std=c++17", "-fPIC", "-Wall", "-I", os.path.join(ROOT, "include")]

@@ -553,6 +553,26 @@ void apply_member(itp2d_ctx* c, const MemberTables& mt, const void* src, void* d
 	kinetic_row<R>(c, mt, dst, dst, acc, vlast, 1, 0);
 }
 
+// The whole step in one launch where the grid is small and square.
+template <class R>
+bool propagate_small(itp2d_ctx* c) {
+	if (c->boundary != ITP2D_PERIODIC || c->sx != c->sy || c->m > 8) return false;
+	SmallStepArgs a = {};
+	a.psi = c->psi;
+	a.out = c->m == 1 ? c->psi : c->acc;
+	a.tw = plan(c, 0, 0).fft.tw;
+	a.m = c->m;
+	for (int t = 0; t < c->m; t++) {
+		const MemberTables& mt = c->members[t];
+		a.member[t] = {c->null_pot ? nullptr : mt.vh, mt.vsq, c->null_pot ? nullptr : mt.vp,
+				c->B == 0 ? mt.kmul : nullptr, mt.kx, mt.ky};
+	}
+	if (!launch_small_step<R>(a, c->sx, c->k, c->stream)) return false;
+	c->launches++;
+	if (c->m > 1) std::swap(c->psi, c->acc);
+	return true;
+}
+
 // Multi-product propagation (MultiProductSplit over OperatorSum,
 // operatorsum.cpp:61-86): member 1 goes out of place into acc; each later
 // member reads the original psi and its last row pass adds into acc, so the
@@ -562,6 +582,7 @@ template <class R>
 int propagate_fused(itp2d_ctx* c) {
 	const int kind = c->boundary == ITP2D_PERIODIC ? 0 : 1;
 	const LinePlan& ly = plan(c, 1, kind);
+	if (propagate_small<R>(c)) return ITP2D_OK;
 	if (c->m == 1) {
 		apply_member<R>(c, c->members[0], c->psi, c->psi, nullptr);
 		return ITP2D_OK;

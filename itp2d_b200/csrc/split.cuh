@@ -121,6 +121,24 @@ template <class R> bool launch_col_pass_reg(const ColPassArgs& a, int k, cudaStr
 // The same for Dirichlet lines (sine transforms, lines_dst.cuh).
 template <class R> bool launch_row_pass_sine(const RowPassArgs& a, int k, cudaStream_t s);
 template <class R> bool launch_col_pass_sine(const ColPassArgs& a, int k, cudaStream_t s);
+// A whole step of k states on an n x n periodic grid in one launch
+// (lines_small.cuh): out = sum of the members applied to psi (out may equal psi
+// where m == 1). Null tables skip a multiply; kmul null: the 1-D ky. Returns
+// false, launching nothing, where it does not apply.
+struct SmallMember {
+	const void *vh, *vsq, *vp;    // first, interior and last potential exponential
+	const void *kmul, *kx, *ky;   // as in RowPassArgs / ColPassArgs
+};
+struct SmallStepArgs {
+	const void* psi;
+	void* out;
+	const void* tw;
+	int m;
+	SmallMember member[8];
+};
+template <class R> bool launch_small_step(const SmallStepArgs& a, int n, int k, cudaStream_t s);
+template <> bool launch_small_step<double>(const SmallStepArgs&, int, int, cudaStream_t);
+template <> bool launch_small_step<float>(const SmallStepArgs&, int, int, cudaStream_t);
 // Register-FFT energy passes; their tile sizes are energy_row_tile_reg rows
 // (of k states' sy rows) and energy_col_tile_reg columns, 0 for lines they do
 // not take.
