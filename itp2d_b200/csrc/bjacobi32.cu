@@ -2,15 +2,18 @@
 //
 // The FP32 form's overlap is accurate to about 1e-5 (split-BF16 tensor-core
 // contraction) and its eigensolve stops at a largest rotation tangent of 1e-3,
-// so FP64 arithmetic buys nothing there. This is the schedule of bjacobi.cu —
-// round-robin pairs of 16-index blocks, 32 x 32 subproblems swept by one CTA
-// per pair (k_p / 32 of them; cross pairs only except every 16th round),
-// phase 1 of round t pipelined against phase 2 of round t - 1 (here on four
-// 128-thread groups per CTA), one grid barrier per round — in single
-// precision: the rotation set-up uses the hardware square root and reciprocal
-// square root directly (no Newton refinement), and the block products are
-// FFMA. Its latency chains are the short ones of FP32, which is what the
-// latency-bound subproblem sweeps need.
+// so FP64 arithmetic buys nothing there. The schedule and the inner sweeps are
+// those of bjacobi.cu (in single precision), with block products in FFMA: four
+// groups of 128 threads per CTA, each on its own item of phase 2 with the next
+// item's operands in flight (cp.async, two stages).
+//
+// Before, the sweeps kept all of M and Q in shared memory with two barriers
+// per full round, every block of A was formed (not the upper triangle only),
+// and an item's loads and products came one after the other; whole solves then
+// and now: 3.54 and 2.63 ms at k = 500 (7 sweeps), 17.0 and 11.3 ms at k = 1000
+// (8), 120 and 73 ms at k = 2000 (9). At k = 500 a round is 12 us: 2.5 forming
+// the subproblem, 6.2 in its sweep (760 cycles per inner round, the rotation and
+// the update of M about as long as each other) and 1.3 in the grid barrier.
 //
 // Accuracy: rotations are unitary to a few FP32 units, so the eigenvector
 // matrix is orthonormal to about 1e-6; normalize_columns_kernel (jacobi.cu)
@@ -20,6 +23,7 @@
 #include <cooperative_groups.h>
 
 #include "../../include/itp2d_gpu.h"
+#include "bjacobi.cuh"
 #include "contract.cuh"
 
 namespace cg = cooperative_groups;
@@ -28,244 +32,85 @@ namespace itp2d {
 
 namespace {
 
-constexpr int BS = 16;        // block size
-constexpr int MS = 32;        // subproblem size: two blocks
-constexpr int NR = MS / 2;    // rotations per inner round
-// Row pitch 48 floats: rows p and p + 1 fall 16 banks apart, so the half-warps
-// of the cross-pair updates (consecutive p, 16 consecutive columns) and of the
-// block products (two consecutive rows per warp) never share a bank.
-constexpr int LD = 48;
-constexpr int PL = MS * LD;   // floats per plane
-// 512 threads, one CTA per SM: in an inner round, threads [0, 256) update the
-// 256 2 x 2 blocks of M while threads [256, 512) rotate the columns of Q.
-constexpr int kThreads = 512;
-constexpr int kMThreads = NR * NR;
-// Phase 2 runs on four groups of 128 threads, each on its own block product:
-// four DRAM-latency-bound products in flight per SM.
+using namespace bj;
+
+// Row pitch of the operands: 16-byte rows for cp.async, and column reads of
+// eight rows (the mirrored half of a product) spread over the banks.
+constexpr int LD = MS + 2;
+constexpr int OP = MS * LD;
 constexpr int kGroups = 4;
 constexpr int kGT = kThreads / kGroups;
-constexpr int kFullEvery = 16;
 constexpr float kSkipRel = 1e-7f;
 constexpr float kNoiseRel = 1e-6f;
 
-__device__ __forceinline__ int rr_player(int pos, int r, int npos) {
-	return pos == 0 ? 0 : ((pos - 1 + r) % (npos - 1)) + 1;
-}
-
-__device__ __forceinline__ int gidx(int i, int P, int Q) { return i < BS ? P * BS + i : Q * BS + (i - BS); }
-
 struct Shared32 {
-	// phase 1: [0,1] M, [2,3] Q, [4,5] formation operands; phase 2: group g
-	// of the CTA uses [6g, 6g + 6): X/T, Q_r, Q_c
-	float pl[6 * kGroups][PL];
-	// rotations of two consecutive inner rounds (round r in buffer r & 1)
-	float4 rot[2][NR];  // rotation j: (sin, tau, Re e, Im e)
-	float rap[2][NR], raq[2][NR];  // M(p, p), M(q, q) after the round
-	int rpq[2][NR];     // p | q << 8 | applied << 16
+	// phase 1: op[0..2] formation operands, then two buffers of M and the Q
+	// warps' exchange area; phase 2: group g uses op[6 g, 6 g + 6), two stages of
+	// (X, Q_c, Q_r), all with element (m, l) at [m * LD + l]
+	float2 op[6 * kGroups][OP];
+	float2 rst[2][NR];  // (sin, tau), (0, 0): none
+	float2 re[2][NR];   // e = c / |c|
 	int next[kGroups];  // phase-2 item of each thread group
 	int cnt;
 	unsigned long long tmax;  // bits of a non-negative double
+	__device__ float2* m(int b) { return op[3] + b * OP; }
+	__device__ float2* xch() { return op[5]; }
 };
 
-// Rotation j of an inner round (into rotation buffer buf) of the local pair
-// (p, q) with M(p, p) = a, M(q, q) = b, M(p, q) = (cr, ci): with
-// d = (b - a) / 2, r = sqrt(d^2 + |c|^2), u = |d| + r and w = 2 r u:
-// cos = u / sqrt(w), |sin| = |c| / sqrt(w), tau = |sin| / (1 + cos),
-// tan = |c| / u (the formulas of bjacobi.cu).
-__device__ __forceinline__ void inner_rotation32(Shared32& sh, int buf, int j, int p, int q, float a, float b,
-		float cr, float ci, int& cnt, float& tmax) {
-	const float c2 = cr * cr + ci * ci;
-	const float scale2 = fabsf(a) * fabsf(b);
-	if (!(c2 > 0.f && c2 > kSkipRel * kSkipRel * scale2)) {
-		sh.rap[buf][j] = a;
-		sh.raq[buf][j] = b;
-		sh.rpq[buf][j] = p | q << 8;
-		return;
-	}
-	const float d = 0.5f * (b - a);
-	const float ad = fabsf(d);
-	const float rn = sqrtf(fmaf(d, d, c2));
-	const float un = ad + rn;
-	const float wn = 2.f * rn * un;
-	const float qn = rsqrtf(wn);
-	const float cabs = sqrtf(c2);
-	const float t = __fdividef(cabs, un);
-	const float ic = rsqrtf(c2);
-	const float sg = d < 0.f ? -1.f : 1.f;
-	sh.rot[buf][j] = make_float4(sg * cabs * qn, sg * __fdividef(cabs, wn * qn + un), cr * ic, ci * ic);
-	sh.rap[buf][j] = a - sg * t * cabs;
-	sh.raq[buf][j] = b + sg * t * cabs;
-	sh.rpq[buf][j] = p | q << 8 | 1 << 16;
-	if (c2 > kNoiseRel * kNoiseRel * scale2) {
-		cnt++;
-		tmax = fmaxf(tmax, t);
-	}
+// c += a b, c += conj(a) b
+template <bool CONJ>
+__device__ __forceinline__ void cfma(float2& c, float2 a, float2 b) {
+	const float ai = CONJ ? -a.y : a.y;
+	c.x = fmaf(a.x, b.x, fmaf(-ai, b.y, c.x));
+	c.y = fmaf(a.x, b.y, fmaf(ai, b.x, c.y));
 }
+__device__ __forceinline__ float4 ld4(const float2* p) { return *reinterpret_cast<const float4*>(p); }
 
-// Rotation j of an inner round from the subproblem in shared memory.
-__device__ __forceinline__ void inner_rotation32_sm(Shared32& sh, int buf, int j, int p, int q, int& cnt,
-		float& tmax) {
-	const float* mr = sh.pl[0];
-	const float* mi = sh.pl[1];
-	inner_rotation32(sh, buf, j, p, q, mr[p * LD + p], mr[q * LD + q], mr[p * LD + q], mi[p * LD + q], cnt, tmax);
+// 32 x 32 products of one thread group: thread lt has rows r0 .. r0 + 3 and
+// columns c0 and c0 + 16 (group_at); per step a warp reads its rows by broadcast
+// and its columns in whole 128-byte rows.
+__device__ __forceinline__ void group_at(int lt, int& r0, int& c0) {
+	r0 = 8 * (lt >> 5) + 4 * ((lt >> 4) & 1);
+	c0 = lt & 15;
 }
-
-__device__ __forceinline__ void rows2f(float s, float tau, float er, float ei, float& xpr, float& xpi, float& xqr,
-		float& xqi) {
-	const float ypr = xpr - s * (er * xqr - ei * xqi + tau * xpr);
-	const float ypi = xpi - s * (er * xqi + ei * xqr + tau * xpi);
-	const float yqr = xqr + s * (er * xpr + ei * xpi - tau * xqr);
-	const float yqi = xqi + s * (er * xpi - ei * xpr - tau * xqi);
-	xpr = ypr; xpi = ypi; xqr = yqr; xqi = yqi;
-}
-
-__device__ __forceinline__ void cols2f(float s, float tau, float er, float ei, float& xsr, float& xsi, float& xtr,
-		float& xti) {
-	const float ysr = xsr - s * (er * xtr + ei * xti + tau * xsr);
-	const float ysi = xsi - s * (er * xti - ei * xtr + tau * xsi);
-	const float ytr = xtr + s * (er * xsr - ei * xsi - tau * xtr);
-	const float yti = xti + s * (er * xsi + ei * xsr - tau * xti);
-	xsr = ysr; xsi = ysi; xtr = ytr; xti = yti;
-}
-
-// One inner sweep (full: MS - 1 rounds over all pairs; cross: BS rounds of the
-// BS x BS cross pairs, round r pairing p < BS with BS + (p + r) % BS) on the
-// subproblem in planes 0/1, Q in planes 2/3. In each round the M blocks and
-// the Q columns are rotated by separate threads at the same time.
-// In a cross sweep, round r + 1 pairs p with q' = BS + (p + r + 1) % BS, the
-// second index of pair p + 1 in round r; so the thread updating the block
-// (pair p, pair p + 1) of round r holds M(p, q') and finds M(p, p) and
-// M(q', q') among round r's results, and sets up rotation p of round r + 1
-// right away: one barrier per inner round.
-__device__ void inner_sweep32(Shared32& sh, bool full) {
-	float* mr = sh.pl[0];
-	float* mi = sh.pl[1];
-	float* qr = sh.pl[2];
-	float* qi = sh.pl[3];
-	const int tid = threadIdx.x;
-	const int rounds = full ? MS - 1 : BS;
-	int cnt = 0;
-	float tmax = 0.f;
-	if (tid < NR) {
-		const int p = full ? rr_player(tid, 0, MS) : tid;
-		const int q = full ? rr_player(MS - 1 - tid, 0, MS) : BS + tid;
-		inner_rotation32_sm(sh, 0, tid, p, q, cnt, tmax);
-	}
-	__syncthreads();
-	for (int r = 0; r < rounds; r++) {
-		const int cur = r & 1;
-		if (full && r > 0) {
-			if (tid < NR) inner_rotation32_sm(sh, cur, tid, rr_player(tid, r, MS), rr_player(MS - 1 - tid, r, MS), cnt,
-					tmax);
-			__syncthreads();
-		}
-		if (tid < kMThreads) {
-			const int ja = tid / NR, jb = tid % NR;
-			const int pa = sh.rpq[cur][ja], pb = sh.rpq[cur][jb];
-			const bool ra = pa >> 16, rb = pb >> 16;
-			const bool nx = !full && r + 1 < rounds && jb == ((ja + 1) & (NR - 1));
-			const int p = pa & 255, q = (pa >> 8) & 255, s2 = pb & 255, t2 = (pb >> 8) & 255;
-			if (ja == jb) {
-				if (ra) {
-					mr[p * LD + p] = sh.rap[cur][ja]; mi[p * LD + p] = 0.f;
-					mr[q * LD + q] = sh.raq[cur][ja]; mi[q * LD + q] = 0.f;
-					mr[p * LD + q] = 0.f; mi[p * LD + q] = 0.f;
-					mr[q * LD + p] = 0.f; mi[q * LD + p] = 0.f;
-				}
-			} else if (ra || rb || nx) {
-				float psr = mr[p * LD + s2], psi = mi[p * LD + s2], ptr = mr[p * LD + t2], pti = mi[p * LD + t2];
-				float qsr = mr[q * LD + s2], qsi = mi[q * LD + s2], qtr = mr[q * LD + t2], qti = mi[q * LD + t2];
-				if (ra) {
-					const float4 R = sh.rot[cur][ja];
-					rows2f(R.x, R.y, R.z, R.w, psr, psi, qsr, qsi);
-					rows2f(R.x, R.y, R.z, R.w, ptr, pti, qtr, qti);
-				}
-				if (rb) {
-					const float4 R = sh.rot[cur][jb];
-					cols2f(R.x, R.y, R.z, R.w, psr, psi, ptr, pti);
-					cols2f(R.x, R.y, R.z, R.w, qsr, qsi, qtr, qti);
-				}
-				if (ra || rb) {
-					mr[p * LD + s2] = psr; mi[p * LD + s2] = psi; mr[p * LD + t2] = ptr; mi[p * LD + t2] = pti;
-					mr[q * LD + s2] = qsr; mi[q * LD + s2] = qsi; mr[q * LD + t2] = qtr; mi[q * LD + t2] = qti;
-				}
-				if (nx)
-					inner_rotation32(sh, cur ^ 1, ja, p, t2, sh.rap[cur][ja], sh.raq[cur][jb], ptr, pti, cnt, tmax);
-			}
-		} else {
-			for (int e = tid - kMThreads; e < MS * NR; e += kThreads - kMThreads) {
-				const int i = e / NR, j = e % NR;
-				const int pj = sh.rpq[cur][j];
-				if (!(pj >> 16)) continue;
-				const int p = pj & 255, q = (pj >> 8) & 255;
-				float ysr = qr[i * LD + p], ysi = qi[i * LD + p], ytr = qr[i * LD + q], yti = qi[i * LD + q];
-				const float4 R = sh.rot[cur][j];
-				cols2f(R.x, R.y, R.z, R.w, ysr, ysi, ytr, yti);
-				qr[i * LD + p] = ysr; qi[i * LD + p] = ysi; qr[i * LD + q] = ytr; qi[i * LD + q] = yti;
-			}
-		}
-		__syncthreads();
-	}
-	// counts and tangents of every thread that set up rotations
-	for (int o = 16; o > 0; o >>= 1) {
-		cnt += __shfl_xor_sync(0xffffffffu, cnt, o);
-		tmax = fmaxf(tmax, __shfl_xor_sync(0xffffffffu, tmax, o));
-	}
-	if ((tid & 31) == 0 && cnt) {
-		atomicAdd(&sh.cnt, cnt);
-		atomicMax(&sh.tmax, (unsigned long long)__double_as_longlong((double)tmax));
-	}
-}
-
-// Complex products of 32-deep operands given as plane pairs, FFMA: the thread
-// accumulates rows row0 + r * rstep (r < NRW) by columns col0 + c * cstep
-// (c < NCL). A element (i, m) at a_re[i * as_i + m * as_m], B element (m, l)
-// at b_re[m * LD + l]; conjA conjugates A.
-template <int NRW, int NCL>
-__device__ __forceinline__ void cmm32(const float* ar, const float* ai, int as_i, int as_m, bool conjA,
-		const float* br, const float* bi, int row0, int rstep, int col0, int cstep, float (&cr)[NRW][NCL],
-		float (&ci)[NRW][NCL]) {
+// A B
+__device__ __forceinline__ void group_ab(const float2* A, const float2* B, int r0, int c0, float2 (&c)[4][2]) {
 #pragma unroll
-	for (int r = 0; r < NRW; r++)
-#pragma unroll
-		for (int c = 0; c < NCL; c++) cr[r][c] = ci[r][c] = 0.f;
+	for (int r = 0; r < 4; r++) c[r][0] = c[r][1] = make_float2(0.f, 0.f);
 #pragma unroll 4
-	for (int m = 0; m < MS; m++) {
-		float xr[NRW], xi[NRW], yr[NCL], yi[NCL];
+	for (int m = 0; m < MS; m += 2) {
+		float4 a[4];
+		float2 b[2][2];
 #pragma unroll
-		for (int r = 0; r < NRW; r++) {
-			const int o = (row0 + r * rstep) * as_i + m * as_m;
-			xr[r] = ar[o];
-			xi[r] = conjA ? -ai[o] : ai[o];
-		}
+		for (int r = 0; r < 4; r++) a[r] = ld4(A + (r0 + r) * LD + m);
 #pragma unroll
-		for (int c = 0; c < NCL; c++) {
-			yr[c] = br[m * LD + col0 + c * cstep];
-			yi[c] = bi[m * LD + col0 + c * cstep];
-		}
+		for (int u = 0; u < 2; u++)
 #pragma unroll
-		for (int r = 0; r < NRW; r++)
+			for (int q = 0; q < 2; q++) b[u][q] = B[(m + u) * LD + c0 + 16 * q];
 #pragma unroll
-			for (int c = 0; c < NCL; c++) {
-				cr[r][c] = fmaf(xr[r], yr[c], fmaf(-xi[r], yi[c], cr[r][c]));
-				ci[r][c] = fmaf(xr[r], yi[c], fmaf(xi[r], yr[c], ci[r][c]));
+		for (int r = 0; r < 4; r++)
+#pragma unroll
+			for (int q = 0; q < 2; q++) {
+				cfma<false>(c[r][q], make_float2(a[r].x, a[r].y), b[0][q]);
+				cfma<false>(c[r][q], make_float2(a[r].z, a[r].w), b[1][q]);
 			}
 	}
 }
-
-// Group products of phase 2: thread lt of 128, warp lw = lt >> 5 owns rows
-// 8 lw .. 8 lw + 7; lane (h, l) computes rows 8 lw + h + 2r at columns l + 16c.
-__device__ __forceinline__ void group_rc(int lt, int r, int c, int& row, int& col) {
-	const int lane = lt & 31, lw = lt >> 5;
-	row = 8 * lw + (lane >> 4) + 2 * r;
-	col = (lane & 15) + 16 * c;
-}
-
-__device__ __forceinline__ void group_gemm(int lt, const float* ar, const float* ai, int as_i, int as_m, bool conjA,
-		const float* br, const float* bi, float (&cr)[4][2], float (&ci)[4][2]) {
-	int row0, col0;
-	group_rc(lt, 0, 0, row0, col0);
-	cmm32<4, 2>(ar, ai, as_i, as_m, conjA, br, bi, row0, 2, col0, 16, cr, ci);
+// A^H B
+__device__ __forceinline__ void group_ahb(const float2* A, const float2* B, int r0, int c0, float2 (&c)[4][2]) {
+#pragma unroll
+	for (int r = 0; r < 4; r++) c[r][0] = c[r][1] = make_float2(0.f, 0.f);
+#pragma unroll 8
+	for (int m = 0; m < MS; m++) {
+		const float4 a0 = ld4(A + m * LD + r0), a1 = ld4(A + m * LD + r0 + 2);
+		const float2 a[4] = {make_float2(a0.x, a0.y), make_float2(a0.z, a0.w), make_float2(a1.x, a1.y),
+				make_float2(a1.z, a1.w)};
+		const float2 b[2] = {B[m * LD + c0], B[m * LD + c0 + 16]};
+#pragma unroll
+		for (int r = 0; r < 4; r++)
+#pragma unroll
+			for (int q = 0; q < 2; q++) cfma<true>(c[r][q], a[r], b[q]);
+	}
 }
 
 // Barrier of one thread group (named barrier 1 + g, 128 threads).
@@ -273,26 +118,18 @@ __device__ __forceinline__ void group_sync(int g) {
 	asm volatile("bar.sync %0, %1;\n" ::"r"(1 + g), "r"(kGT) : "memory");
 }
 
-__device__ __forceinline__ int rr_position(int p, int r, int npos) {
-	if (p == 0) return 0;
-	const int m = npos - 1;
-	return ((p - 1 - r) % m + m) % m + 1;
-}
-
-// Phase 1 for pair j of round t (bjacobi.cu phase1_item in FP32).
+// Phase 1 for pair j of round t (bjacobi.cu phase1_item in FP32; Q is kept as
+// Q(i, l) at [i * MS + l] here).
 __device__ void phase1_item32(Shared32& sh, int j, long long t, int rounds, int nb, int np, int kp,
 		const float2* prev, const float2* prev2, const float2* Qprev, float2* Qout, float2* out) {
 	const int tid = threadIdx.x;
 	const int rr = (int)(t % rounds);
 	const int P = rr_player(j, rr, nb), Q = rr_player(nb - 1 - j, rr, nb);
-	float* mr = sh.pl[0];
-	float* mi = sh.pl[1];
+	float2* M = sh.m(0);
 	if (t == 0) {
 		for (int e = tid; e < MS * MS; e += kThreads) {
 			const int i = e / MS, l = e % MS;
-			const float2 v = __ldcg(prev + (long long)gidx(i, P, Q) * kp + gidx(l, P, Q));
-			mr[i * LD + l] = v.x;
-			mi[i * LD + l] = v.y;
+			M[i * LDM + l] = __ldcg(prev + (long long)gidx(i, P, Q) * kp + gidx(l, P, Q));
 		}
 	} else {
 		const int ro = (int)((t - 1) % rounds);
@@ -317,158 +154,158 @@ __device__ void phase1_item32(Shared32& sh, int j, long long t, int rounds, int 
 			const int g0 = (half ? Q : P) * BS;
 			ldg[it] = __ldcg(prev + (long long)(g0 + i) * kp + g0 + l);
 		}
+		float2 *X = sh.op[0], *Ta = sh.op[1], *Tb = sh.op[2];
 #pragma unroll
 		for (int it = 0; it < NL; it++) {
-			const int e = it * kThreads + tid, i = e / MS, l = e % MS;
-			mr[i * LD + l] = la[it].x;
-			mi[i * LD + l] = la[it].y;
-			sh.pl[2][i * LD + l] = lqa[it].x;
-			sh.pl[3][i * LD + l] = lqa[it].y;
-			sh.pl[4][i * LD + l] = lqb[it].x;
-			sh.pl[5][i * LD + l] = lqb[it].y;
+			const int e = it * kThreads + tid, o = (e / MS) * LD + e % MS;
+			X[o] = la[it];
+			Ta[o] = lqa[it];
+			Tb[o] = lqb[it];
 		}
 		__syncthreads();
 		// only the (hP, hQ) quadrant of Q_a^H A_{t-2}(a, b) Q_b enters the
-		// subproblem: T = A_{t-2}(a, b) Q_b[:, hQ half] (32 x 16, one element per
-		// thread), then C = Q_a[:, hP half]^H T (16 x 16, threads [0, 256))
-		{
-			const int lane = tid & 31, warp = tid >> 5;
-			const int trow = 2 * warp + (lane >> 4), tcol = lane & 15;
-			float tr[1][1], ti[1][1];
-			cmm32<1, 1>(sh.pl[0], sh.pl[1], LD, 1, false, sh.pl[4], sh.pl[5], trow, 0, hQ * BS + tcol, 0, tr, ti);
-			__syncthreads();
-			mr[trow * LD + tcol] = tr[0][0];
-			mi[trow * LD + tcol] = ti[0][0];
-			__syncthreads();
-			float cr[1][1], ci[1][1];
-			const int i = (tid >> 4) & (BS - 1), l = tid & 15;
-			if (tid < BS * BS)
-				cmm32<1, 1>(sh.pl[2] + hP * BS, sh.pl[3] + hP * BS, 1, LD, true, sh.pl[0], sh.pl[1], i, 0, l, 0, cr,
-						ci);
-			__syncthreads();
-			if (tid < BS * BS) {
-				mr[i * LD + BS + l] = cr[0][0];
-				mi[i * LD + BS + l] = ci[0][0];
-				mr[(BS + l) * LD + i] = cr[0][0];
-				mi[(BS + l) * LD + i] = -ci[0][0];
+		// subproblem: T = A_{t-2}(a, b) Q_b[:, hQ half] (32 x 16, threads [0, 256)
+		// two rows each), then C = Q_a[:, hP half]^H T (16 x 16, threads [0, 256))
+		const int row = tid >> 4, col = tid & 15;
+		if (tid < BS * BS) {
+			float2 c0 = make_float2(0.f, 0.f), c1 = c0;
+#pragma unroll 8
+			for (int m = 0; m < MS; m += 2) {
+				const float4 a0 = ld4(X + row * LD + m), a1 = ld4(X + (row + BS) * LD + m);
+				const float2 b0 = Tb[m * LD + hQ * BS + col], b1 = Tb[(m + 1) * LD + hQ * BS + col];
+				cfma<false>(c0, make_float2(a0.x, a0.y), b0);
+				cfma<false>(c1, make_float2(a1.x, a1.y), b0);
+				cfma<false>(c0, make_float2(a0.z, a0.w), b1);
+				cfma<false>(c1, make_float2(a1.z, a1.w), b1);
 			}
+			// T beside the other half of Q_b, which nothing reads any more
+			float2* T = Tb + (hQ ^ 1) * BS + col;
+			T[row * LD] = c0;
+			T[(row + BS) * LD] = c1;
 		}
+		__syncthreads();
+		if (tid < BS * BS) {
+			const float2* T = Tb + (hQ ^ 1) * BS + col;
+			float2 c = make_float2(0.f, 0.f);
+#pragma unroll 8
+			for (int m = 0; m < MS; m++) cfma<true>(c, Ta[m * LD + hP * BS + row], T[m * LD]);
+			M[row * LDM + BS + col] = c;
+		}
+		// diagonal blocks (P, P) and (Q, Q) of A_{t-1}
 #pragma unroll
 		for (int it = 0; it < ND; it++) {
 			const int e = it * kThreads + tid;
 			const int half = e / (BS * BS), i = (e / BS) % BS, l = e % BS;
-			mr[(half * BS + i) * LD + half * BS + l] = ldg[it].x;
-			mi[(half * BS + i) * LD + half * BS + l] = ldg[it].y;
+			M[(half * BS + i) * LDM + half * BS + l] = ldg[it];
 		}
 	}
-	for (int e = tid; e < MS * MS; e += kThreads) {
-		const int i = e / MS, l = e % MS;
-		sh.pl[2][i * LD + l] = (i == l) ? 1.f : 0.f;
-		sh.pl[3][i * LD + l] = 0.f;
-	}
 	__syncthreads();
-	inner_sweep32(sh, rr % kFullEvery == 0);
 	float2* Qg = Qout + (size_t)j * MS * MS;
+	const bool full = rr % kFullEvery == 0;
+	if (full) inner_sweep<float, true, false>(sh, kSkipRel, kNoiseRel, Qg);
+	else inner_sweep<float, false, false>(sh, kSkipRel, kNoiseRel, Qg);
+	const int last = full ? (MS - 1) & 1 : BS & 1;
 	for (int e = tid; e < MS * MS; e += kThreads) {
 		const int i = e / MS, l = e % MS;
-		Qg[e] = make_float2(sh.pl[2][i * LD + l], sh.pl[3][i * LD + l]);
-		out[(long long)gidx(i, P, Q) * kp + gidx(l, P, Q)] = make_float2(mr[i * LD + l], mi[i * LD + l]);
+		const float2 v = ld_m(sh.m(last), i, l);
+		out[(long long)gidx(i, P, Q) * kp + gidx(l, P, Q)] = make_float2(v.x, i == l ? 0.f : v.y);
 	}
 	__syncthreads();
 }
 
-// Phase 2 item w of round ro (bjacobi.cu phase2_item in FP32), on one thread
-// group of the CTA, with its own planes and named barrier.
-__device__ void phase2_item32(Shared32& sh, int g, int w, int ro, int nb, int np, int kp, const float2* src,
-		float2* dst, float2* V, const float2* Qr) {
-	const int lt = threadIdx.x & (kGT - 1);
-	float* xr = sh.pl[6 * g + 0];
-	float* xi = sh.pl[6 * g + 1];
-	float* ar = sh.pl[6 * g + 2];
-	float* ai = sh.pl[6 * g + 3];
-	float* br = sh.pl[6 * g + 4];
-	float* bi = sh.pl[6 * g + 5];
-	const int nA2 = np * (np - 1);
-	constexpr int NH = MS * MS / kGT;  // elements per thread and operand
-	float cr[4][2], ci[4][2];
-	if (w < nA2) {
-		const int jr = w / (np - 1);
-		int jc = w % (np - 1);
-		if (jc >= jr) jc++;
-		const int Pr = rr_player(jr, ro, nb), Qr_ = rr_player(nb - 1 - jr, ro, nb);
-		const int Pc = rr_player(jc, ro, nb), Qc = rr_player(nb - 1 - jc, ro, nb);
-		// all global loads of the item at once, then the shared-memory stores
-		float2 lx[NH], la[NH], lb[NH];
+// Starts the copies of an item's operands into stage st by one group.
+__device__ __forceinline__ void phase2_fetch32(float2 (*st)[OP], const Item& it, int lt, int ro, int nb, int kp,
+		const float2* src, const float2* V, const float2* Qr) {
+	const int Pc = rr_player(it.jc, ro, nb), Qc = rr_player(nb - 1 - it.jc, ro, nb);
+	const int Pr = it.is_v ? 2 * it.jr : rr_player(it.jr, ro, nb);
+	const int Qr_ = it.is_v ? 2 * it.jr + 1 : rr_player(nb - 1 - it.jr, ro, nb);
+	const float2* X = it.is_v ? V : src;
+	auto cp = [](float2* dst, const float2* s) {
+		asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"((unsigned)__cvta_generic_to_shared(dst)),
+				"l"(s) : "memory");
+	};
 #pragma unroll
-		for (int it = 0; it < NH; it++) {
-			const int e = it * kGT + lt, i = e / MS, l = e % MS;
-			lx[it] = __ldcg(src + (long long)gidx(i, Pr, Qr_) * kp + gidx(l, Pc, Qc));
-			la[it] = __ldcg(Qr + (size_t)jr * MS * MS + e);
-			lb[it] = __ldcg(Qr + (size_t)jc * MS * MS + e);
-		}
-#pragma unroll
-		for (int it = 0; it < NH; it++) {
-			const int e = it * kGT + lt, o = (e / MS) * LD + e % MS;
-			xr[o] = lx[it].x;
-			xi[o] = lx[it].y;
-			ar[o] = la[it].x;
-			ai[o] = la[it].y;
-			br[o] = lb[it].x;
-			bi[o] = lb[it].y;
-		}
-		group_sync(g);
-		group_gemm(lt, xr, xi, LD, 1, false, br, bi, cr, ci);  // T = X Qc
-		group_sync(g);
-#pragma unroll
-		for (int r = 0; r < 4; r++)
-#pragma unroll
-			for (int c = 0; c < 2; c++) {
-				int row, col;
-				group_rc(lt, r, c, row, col);
-				xr[row * LD + col] = cr[r][c];
-				xi[row * LD + col] = ci[r][c];
-			}
-		group_sync(g);
-		group_gemm(lt, ar, ai, 1, LD, true, xr, xi, cr, ci);  // Qr^H T
-#pragma unroll
-		for (int r = 0; r < 4; r++)
-#pragma unroll
-			for (int c = 0; c < 2; c++) {
-				int row, col;
-				group_rc(lt, r, c, row, col);
-				dst[(long long)gidx(row, Pr, Qr_) * kp + gidx(col, Pc, Qc)] = make_float2(cr[r][c], ci[r][c]);
-			}
-	} else {
-		const int v = w - nA2;
-		const int rb = v / np, jc = v % np;
-		const int Pc = rr_player(jc, ro, nb), Qc = rr_player(nb - 1 - jc, ro, nb);
-		float2 lx[NH], lb[NH];
-#pragma unroll
-		for (int it = 0; it < NH; it++) {
-			const int e = it * kGT + lt, i = e / MS, l = e % MS;
-			lx[it] = __ldcg(V + (long long)(rb * MS + i) * kp + gidx(l, Pc, Qc));
-			lb[it] = __ldcg(Qr + (size_t)jc * MS * MS + e);
-		}
-#pragma unroll
-		for (int it = 0; it < NH; it++) {
-			const int e = it * kGT + lt, o = (e / MS) * LD + e % MS;
-			xr[o] = lx[it].x;
-			xi[o] = lx[it].y;
-			br[o] = lb[it].x;
-			bi[o] = lb[it].y;
-		}
-		group_sync(g);
-		group_gemm(lt, xr, xi, LD, 1, false, br, bi, cr, ci);  // V Qc
-#pragma unroll
-		for (int r = 0; r < 4; r++)
-#pragma unroll
-			for (int c = 0; c < 2; c++) {
-				int row, col;
-				group_rc(lt, r, c, row, col);
-				V[(long long)(rb * MS + row) * kp + gidx(col, Pc, Qc)] = make_float2(cr[r][c], ci[r][c]);
-			}
+	for (int h = 0; h < MS * MS / 2 / kGT; h++) {
+		const int e = 2 * (h * kGT + lt), i = e / MS, l = e % MS, o = i * LD + l;
+		cp(st[0] + o, X + (long long)gidx(i, Pr, Qr_) * kp + gidx(l, Pc, Qc));
+		cp(st[1] + o, Qr + (size_t)it.jc * MS * MS + e);
+		if (!it.is_v) cp(st[2] + o, Qr + (size_t)it.jr * MS * MS + e);
 	}
+	asm volatile("cp.async.commit_group;\n" ::: "memory");
+}
+
+// The products of an item from stage st, written to dst or V.
+__device__ __forceinline__ void phase2_item32(float2 (*st)[OP], const Item& it, int g, int lt, int ro, int nb, int kp,
+		float2* dst, float2* V) {
+	const int Pc = rr_player(it.jc, ro, nb), Qc = rr_player(nb - 1 - it.jc, ro, nb);
+	int r0, c0;
+	group_at(lt, r0, c0);
+	float2 c[4][2];
+	group_ab(st[0], st[1], r0, c0, c);  // V Q_c, or T = X Q_c
+	if (it.is_v) {
+#pragma unroll
+		for (int r = 0; r < 4; r++)
+#pragma unroll
+			for (int q = 0; q < 2; q++) V[(long long)(it.jr * MS + r0 + r) * kp + gidx(c0 + 16 * q, Pc, Qc)] = c[r][q];
+		return;
+	}
+	const int Pr = rr_player(it.jr, ro, nb), Qr_ = rr_player(nb - 1 - it.jr, ro, nb);
 	group_sync(g);
+#pragma unroll
+	for (int r = 0; r < 4; r++)
+#pragma unroll
+		for (int q = 0; q < 2; q++) st[0][(r0 + r) * LD + c0 + 16 * q] = c[r][q];
+	group_sync(g);
+	group_ahb(st[2], st[0], r0, c0, c);  // Q_r^H T
+#pragma unroll
+	for (int q = 0; q < 2; q++) {
+		const long long gc = gidx(c0 + 16 * q, Pc, Qc), gr = gidx(r0, Pr, Qr_);
+#pragma unroll
+		for (int r = 0; r < 4; r++) dst[(gr + r) * kp + gc] = c[r][q];
+		float4* mirror = reinterpret_cast<float4*>(dst + gc * kp + gr);
+		mirror[0] = make_float4(c[0][q].x, -c[0][q].y, c[1][q].x, -c[1][q].y);
+		mirror[1] = make_float4(c[2][q].x, -c[2][q].y, c[3][q].x, -c[3][q].y);
+	}
+}
+
+// The items of round ro that one group takes (phase2 of bjacobi.cu).
+__device__ void phase2_32(Shared32& sh, int ro, int nb, int np, int nW, int kp, const float2* src, float2* dst,
+		float2* V, const float2* Qr, int* ctr) {
+	const int g = threadIdx.x / kGT, lt = threadIdx.x & (kGT - 1);
+	auto take = [&]() {
+		if (lt == 0) sh.next[g] = atomicAdd(ctr, 1);
+		group_sync(g);
+		const int w = sh.next[g];
+		group_sync(g);
+		return w;
+	};
+	float2(*st)[OP] = sh.op + 6 * g;
+	int w = take(), cur = 0;
+	if (w >= nW) return;
+	Item it = item_of(w, np);
+	phase2_fetch32(st, it, lt, ro, nb, kp, src, V, Qr);
+	int wn = take();
+	while (w < nW) {
+		Item nx{};
+		if (wn < nW) {
+			nx = item_of(wn, np);
+			phase2_fetch32(st + 3 * (cur ^ 1), nx, lt, ro, nb, kp, src, V, Qr);
+			asm volatile("cp.async.wait_group 1;\n" ::: "memory");
+		} else {
+			asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+		}
+		group_sync(g);
+		// the index after next arrives during the products
+		int w2 = nW;
+		if (lt == 0 && wn < nW) w2 = atomicAdd(ctr, 1);
+		phase2_item32(st + 3 * cur, it, g, lt, ro, nb, kp, dst, V);
+		if (lt == 0) sh.next[g] = w2;
+		group_sync(g);  // the stage is free for the item after next
+		it = nx;
+		w = wn;
+		wn = sh.next[g];
+		cur ^= 1;
+	}
 }
 
 // The cooperative solve: bjacobi_kernel of bjacobi.cu in FP32 (one CTA per SM). A_r lives in
@@ -484,7 +321,7 @@ __global__ void __launch_bounds__(kThreads, 1) bjacobi32_kernel(float2* A0, floa
 	const int np = nb / 2;
 	const int rounds = nb - 1;
 	const int nrb = kp / MS;
-	const int nW = np * (np - 1) + nrb * np;
+	const int nW = np * (np - 1) / 2 + nrb * np;
 	float2* const bufs[3] = {A0, A1, A2};
 	const size_t qstride = (size_t)np * MS * MS;
 	const bool split = (int)gridDim.x > np;
@@ -519,21 +356,7 @@ __global__ void __launch_bounds__(kThreads, 1) bjacobi32_kernel(float2* A0, floa
 			const int ro = (int)((t - 1) % rounds);
 			const float2* src = bufs[(t + 2) % 3];
 			float2* dst = bufs[t % 3];
-			// items handed out by the round's counter; the next index is fetched
-			// while the current item is processed
-			const int g = tid / kGT, lt = tid & (kGT - 1);
-			int* ctr = p2ctr + ((t - 1) & 3);
-			if (lt == 0) sh.next[g] = atomicAdd(ctr, 1);
-			group_sync(g);
-			int w = sh.next[g];
-			while (w < nW) {
-				int wn = 0;
-				if (lt == 0) wn = atomicAdd(ctr, 1);
-				phase2_item32(sh, g, w, ro, nb, np, kp, src, dst, V, Qbuf + ((t + 1) & 1) * qstride);
-				if (lt == 0) sh.next[g] = wn;
-				group_sync(g);
-				w = sh.next[g];
-			}
+			phase2_32(sh, ro, nb, np, nW, kp, src, dst, V, Qbuf + ((t + 1) & 1) * qstride, p2ctr + ((t - 1) & 3));
 		}
 		const bool sweep_end = do_p1 && (t % rounds == rounds - 1);
 		if (sweep_end && tid == 0) {
@@ -608,7 +431,9 @@ cudaError_t launch_bjacobi32(const double2* S, int k, JacobiWork& w, int num_sms
 	e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, bjacobi32_kernel, kThreads, smem);
 	if (e != cudaSuccess) return e;
 	if (per_sm < 1) return cudaErrorLaunchOutOfResources;
-	const int blocks = num_sms * std::min(per_sm, 1);
+	// one CTA per phase-1 pair and one per four phase-2 items, at most one per SM
+	const int np = kp / MS, nW = np * (np - 1) / 2 + np * np;
+	const int blocks = std::min(num_sms, np + (nW + kGroups - 1) / kGroups);
 	int kpv = kp, ms = w.max_sweeps;
 	double tau = w.tau_final > 0.0 ? w.tau_final : 1e-3;
 	int* counters = w.counters;

@@ -72,3 +72,26 @@ def test_tiny_coupling_is_resolved(capi):
     ref = np.linalg.eigvalsh(M)
     assert np.max(np.abs(ev - ref)) < 8 * EPS
     assert np.max(np.abs(M @ U - U * ev[None, :])) < 8 * EPS
+
+
+# first size on the single-precision solver, odd sizes, the last of a padding block
+@pytest.mark.parametrize("k", [256, 257, 289, 352])
+def test_single_precision_orthonormalisation(capi, k):
+    n = 64
+    rng = np.random.default_rng(k)
+    dx = 0.2
+    # overlap X diag(l) X^H with eigenvalues in [0.5, 1], one pair 1e-5 apart
+    lam = np.linspace(0.5, 1.0, k)
+    lam[1] = lam[0] + 1e-5
+    X = np.linalg.qr(rng.standard_normal((k, k)) + 1j * rng.standard_normal((k, k)))[0]
+    Y = np.linalg.qr(rng.standard_normal((n * n, k)) + 1j * rng.standard_normal((n * n, k)))[0]
+    psi = ((Y * np.sqrt(lam)) @ X.conj().T).T.reshape(k, n, n) / dx
+    c = capi.Context(n, n, dx, k, precision=capi.FP32)
+    c.upload(psi)
+    c.orthonormalize()
+    out = c.download().reshape(k, -1)
+    c.close()
+    S = out.conj() @ out.T * dx * dx
+    # an element of the overlap and of the rotation is good to about 1e-5; the
+    # rotations left out after the last sweep are below 1e-6, over 0.5
+    assert np.max(np.abs(S - np.eye(k))) < 1e-4
