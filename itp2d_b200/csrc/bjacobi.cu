@@ -126,10 +126,9 @@ __device__ __forceinline__ void half_sync(int half) {
 // subproblem. prev: A_{t-1} (diagonal pair blocks of round t - 1), prev2:
 // A_{t-2}, Qprev: the Q buffer of round t - 1 (t >= 1). For t = 0 the
 // subproblem is read from prev = A_{-1}, the initial matrix.
-__device__ void phase1_item(Shared& sh, int j, long long t, int rounds, int nb, int np, int kp, double tol,
+__device__ void phase1_item(Shared& sh, int j, long long t, int rr, int rounds, int nb, int np, int kp, double tol,
 		const double2* prev, const double2* prev2, const double2* Qprev, double2* Qout, double2* out) {
 	const int tid = threadIdx.x;
-	const int rr = (int)(t % rounds);
 	const int P = rr_player(j, rr, nb), Q = rr_player(nb - 1 - j, rr, nb);
 	double2* M = sh.m(0);
 	if (t == 0) {
@@ -139,7 +138,7 @@ __device__ void phase1_item(Shared& sh, int j, long long t, int rounds, int nb, 
 		}
 	} else {
 		// the round t - 1 pairs (a, b) holding P and Q, and the halves they sit in
-		const int ro = (int)((t - 1) % rounds);
+		const int ro = rr ? rr - 1 : rounds - 1;
 		const int posP = rr_position(P, ro, nb), posQ = rr_position(Q, ro, nb);
 		const int a = posP < np ? posP : nb - 1 - posP, hP = posP < np ? 0 : 1;
 		const int b = posQ < np ? posQ : nb - 1 - posQ, hQ = posQ < np ? 0 : 1;
@@ -364,27 +363,29 @@ __global__ void __launch_bounds__(kThreads, 1) bjacobi_kernel(double2* A0, doubl
 
 	int sweep = 0;
 	bool stop = false, converged = false;
+	// round t, t mod 3 and t mod rounds (64-bit remainders cost 1000 cycles a round)
 	long long t = 0;
+	int t3 = 0, rr = 0;
 	for (;;) {
 		const bool do_p1 = !stop;  // phase 1 of round t
 		// round t + 1's item counter (its last use, round t - 3, is complete)
 		if (blockIdx.x == 0 && tid == 0) p2ctr[(t + 1) & 3] = 0;
 		const bool do_p2 = t >= 1;  // phase 2 of round t - 1
 		if (do_p1 && (int)blockIdx.x < p1) {
-			const double2* prev = bufs[t % 3];
-			const double2* prev2 = bufs[(t + 2) % 3];
-			double2* out = bufs[(t + 1) % 3];
+			const double2* prev = bufs[t3];
+			const double2* prev2 = bufs[t3 == 0 ? 2 : t3 - 1];
+			double2* out = bufs[t3 == 2 ? 0 : t3 + 1];
 			for (int j = blockIdx.x; j < np; j += p1)
-				phase1_item(sh, j, t, rounds, nb, np, kp, tol, prev, prev2, Qbuf + ((t + 1) & 1) * qstride,
+				phase1_item(sh, j, t, rr, rounds, nb, np, kp, tol, prev, prev2, Qbuf + ((t + 1) & 1) * qstride,
 						Qbuf + (t & 1) * qstride, out);
 		}
 		if (do_p2 && ((int)blockIdx.x >= p2first || join)) {
-			const int ro = (int)((t - 1) % rounds);
-			const double2* src = bufs[(t + 2) % 3];
-			double2* dst = bufs[t % 3];
+			const int ro = rr ? rr - 1 : rounds - 1;
+			const double2* src = bufs[t3 == 0 ? 2 : t3 - 1];
+			double2* dst = bufs[t3];
 			phase2(sh, ro, nb, np, nW, kp, src, dst, V, Qbuf + ((t + 1) & 1) * qstride, p2ctr + ((t - 1) & 3));
 		}
-		const bool sweep_end = do_p1 && (t % rounds == rounds - 1);
+		const bool sweep_end = do_p1 && rr == rounds - 1;
 		if (sweep_end && tid == 0) {
 			if (sh.cnt) atomicAdd(&counters[sweep], sh.cnt);
 			if (sh.tmax) atomicMax(&tmax[sweep], sh.tmax);
@@ -405,6 +406,8 @@ __global__ void __launch_bounds__(kThreads, 1) bjacobi_kernel(double2* A0, doubl
 			if (sweep >= max_sweeps) stop = true;
 		}
 		t++;
+		t3 = t3 == 2 ? 0 : t3 + 1;
+		rr = rr == rounds - 1 ? 0 : rr + 1;
 	}
 	// the last round completed is t - 1; A_{t-1} lives in bufs[t % 3]
 	if (blockIdx.x == 0 && tid == 0) {

@@ -22,7 +22,8 @@ constexpr int kFullEvery = 16;
 
 // Round-robin pairing of npos positions (circle method): position 0 fixed.
 __device__ __forceinline__ int rr_player(int pos, int r, int npos) {
-	return pos == 0 ? 0 : ((pos - 1 + r) % (npos - 1)) + 1;
+	const int v = pos - 1 + r;  // 0 <= r < npos - 1
+	return pos == 0 ? 0 : (v >= npos - 1 ? v - npos + 2 : v + 1);
 }
 
 // Global index of local subproblem index i (< 32) for the block pair (P, Q).
@@ -228,30 +229,35 @@ __device__ __forceinline__ void cols2(R s, R tau, R er, R ei, R& xsr, R& xsi,
 // of NR rotations over all pairs (circle method: pair j is (position j,
 // position MS - 1 - j)), or cross, BS rounds (round r pairs j with BS + (j + r)
 // % BS). The result is left in M buffer R & 1 (R rounds) and the unitary Q in
-// Qg (Q(i, l) at [i * MS + l], transposed with QT). Three groups of warps work
+// Qg (Q(i, l) at [i * MS + l], transposed with QT). Four groups of warps work
 // side by side on round r, one barrier per round:
 //  * warp 0 (lane j: pair j) computes rotation r + 1 from M_r and rotation r.
 //    The two indices of pair j of round r + 1 sit in two different pairs A, B
 //    of round r, so its off-diagonal element is one element of the 2 x 2 block
 //    (A, B) rotated by rotation r; its diagonals are lane A's and lane B's,
-//    carried in registers. It also writes the rotated pairs' own 2 x 2 blocks.
+//    carried in registers.
 //  * warps 1, 2, 3 and 5 (one 2 x 2 block of pairs ja < jb per thread, 120 of
 //    128) form J^H M J in the other M buffer: the upper triangle only.
+//  * warp 4 (lane j: pair j) forms the rotated pairs' own 2 x 2 blocks in double
+//    precision (4 % of an eigensolve at k = 200 in place of warp 0 doing it; in
+//    single precision warp 0 is 2 % faster with them than without).
 //  * warps 6, 7, 9-11 and 13-15 hold Q in registers (lane j: the columns of
 //    pair j, four rows per warp) and pass the columns on through shared memory
 //    (shuffles of 64-bit values cost four times as much there: 3.7 cycles per
 //    32-bit shuffle).
-// Warps 4, 8 and 12 stay idle: warp 0 has its scheduler to itself, because its
+// Warps 8 and 12 stay idle: warp 0 has its scheduler almost to itself, because its
 // chain of rotations bounds the round. Before, every warp updating M set up two
-// rotations itself,
-// in double precision, and all of M and Q crossed shared memory: 2390 cycles
-// per cross round against 940 now (1230 per full round).
+// rotations itself, in double precision, and all of M and Q crossed shared
+// memory: 2390 cycles per cross round against about 1000 now (FP32 about 700).
+// Offsets whose order is known in a cross sweep are formed without comparing
+// (with the round counters kept in 32 bits: 8 % of an eigensolve).
 // `sh`: m(b), the buffers of M; rst, re, the rotations; xch(), the exchange area
 // of the Q warps; cnt and tmax.
 template <class R, bool FULL, bool QT, class SH>
 __device__ __forceinline__ void inner_sweep(SH& sh, R tol, R noise, c2<R>* Qg) {
 	using T = c2<R>;
 	constexpr int ROUNDS = FULL ? MS - 1 : BS;
+	constexpr bool OWN_PAIRS = sizeof(R) == 4;  // warp 0 stores its pairs' blocks
 	const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 	// position of pair index j's second member in round r
 	auto second = [](int j, int r) { return FULL ? circle(MS - 1 - j, r) : BS + ((j + r) & (BS - 1)); };
@@ -260,7 +266,7 @@ __device__ __forceinline__ void inner_sweep(SH& sh, R tol, R noise, c2<R>* Qg) {
 		const int j = lane & (NR - 1);
 		int cnt = 0;
 		R tmax = 0.0;
-		int p = first(j, 0), q = second(j, 0);
+		const int p = first(j, 0), q = second(j, 0);
 		R a = sh.m(0)[m_at(p, p)].x, b = sh.m(0)[m_at(q, q)].x;
 		T c = ld_m(sh.m(0), p, q);
 		Rotation<R> ro = make_rotation<R>(a, b, c.x, c.y, tol, noise, cnt, tmax);
@@ -276,12 +282,21 @@ __device__ __forceinline__ void inner_sweep(SH& sh, R tol, R noise, c2<R>* Qg) {
 		const R sa = a_first ? 1.0 : -1.0, sb = b_first ? 1.0 : -1.0;
 		// the block's element offsets and signs of the imaginary parts, formed
 		// one round ahead: x and y the indices that meet, xo and yo their partners
-		int x, y, o11, o21, o12, o22;
+		int o11, o21, o12, o22;
 		unsigned conj;
 		auto block = [&](int r) {
+			if constexpr (!FULL) {
+				// members below and above BS: the order of all but (xo, y) is known
+				const int y = second(B, r), xo = second(A, r);
+				o11 = j * LDM + y;
+				o21 = m_at(xo, y);
+				o12 = m_at(j, B);
+				o22 = B * LDM + xo;
+				conj = (xo > y ? 2u : 0u) | (j > B ? 4u : 0u) | 8u;
+				return;
+			}
 			const int fa = first(A, r), qa = second(A, r), fb = first(B, r), qb = second(B, r);
-			x = a_first ? fa : qa;
-			y = b_first ? fb : qb;
+			const int x = a_first ? fa : qa, y = b_first ? fb : qb;
 			const int xo = a_first ? qa : fa, yo = b_first ? qb : fb;
 			o11 = m_at(x, y);
 			o21 = m_at(xo, y);
@@ -298,17 +313,16 @@ __device__ __forceinline__ void inner_sweep(SH& sh, R tol, R noise, c2<R>* Qg) {
 			T* mn = sh.m(cur ^ 1);
 			T m11 = m[o11], m21 = m[o21], m12 = m[o12], m22 = m[o22];
 			const T ta = sh.rst[cur][A], ea = sh.re[cur][A], tb = sh.rst[cur][B], eb = sh.re[cur][B];
-			// rotation r's own pair, before the loads are used
-			const int po = p, qo = q;
+			// the diagonals after rotation r, before the loads are used
 			rotated_pair(ro, a, b, c.x, c.y);
 			const R ao = a, bo = b;
-			if (lane < NR) {
-				mn[m_at(po, po)] = mk<R>(ao, 0.0);
-				mn[m_at(qo, qo)] = mk<R>(bo, 0.0);
-				st_m(mn, po, qo, c);
+			if (OWN_PAIRS && lane < NR) {
+				const int p = first(j, r), q = second(j, r);
+				mn[p * (LDM + 1)] = mk<R>(ao, 0.0);
+				mn[q * (LDM + 1)] = mk<R>(bo, 0.0);
+				if (FULL) st_m(mn, p, q, c);
+				else mn[p * LDM + q] = c;
 			}
-			p = x;
-			q = y;
 			if (r + 1 < ROUNDS) {
 				if (conj & 1) m11.y = -m11.y;
 				if (conj & 2) m21.y = -m21.y;
@@ -375,17 +389,29 @@ __device__ __forceinline__ void inner_sweep(SH& sh, R tol, R noise, c2<R>* Qg) {
 			if (on) {
 				const T* m = sh.m(cur);
 				T* mn = sh.m(cur ^ 1);
+				// offsets of the block's elements, and which are stored conjugated
 				const int p = first(ja, r), q = second(ja, r), s = first(jb, r), t = second(jb, r);
-				T ps = ld_m(m, p, s), pt = ld_m(m, p, t), qs = ld_m(m, q, s), qt = ld_m(m, q, t);
+				const int ops = FULL ? m_at(p, s) : ja * LDM + jb, opt = FULL ? m_at(p, t) : ja * LDM + t;
+				const int oqs = FULL ? m_at(q, s) : jb * LDM + q, oqt = m_at(q, t);
+				const bool nps = FULL && p > s, npt = FULL && p > t, nqs = !FULL || q > s, nqt = q > t;
+				T ps = m[ops], pt = m[opt], qs = m[oqs], qt = m[oqt];
+				if (nps) ps.y = -ps.y;
+				if (npt) pt.y = -pt.y;
+				if (nqs) qs.y = -qs.y;
+				if (nqt) qt.y = -qt.y;
 				const T ta = sh.rst[cur][ja], ea = sh.re[cur][ja], tb = sh.rst[cur][jb], eb = sh.re[cur][jb];
 				rows2(ta.x, ta.y, ea.x, ea.y, ps.x, ps.y, qs.x, qs.y);
 				rows2(ta.x, ta.y, ea.x, ea.y, pt.x, pt.y, qt.x, qt.y);
 				cols2(tb.x, tb.y, eb.x, eb.y, ps.x, ps.y, pt.x, pt.y);
 				cols2(tb.x, tb.y, eb.x, eb.y, qs.x, qs.y, qt.x, qt.y);
-				st_m(mn, p, s, ps);
-				st_m(mn, p, t, pt);
-				st_m(mn, q, s, qs);
-				st_m(mn, q, t, qt);
+				if (nps) ps.y = -ps.y;
+				if (npt) pt.y = -pt.y;
+				if (nqs) qs.y = -qs.y;
+				if (nqt) qt.y = -qt.y;
+				mn[ops] = ps;
+				mn[opt] = pt;
+				mn[oqs] = qs;
+				mn[oqt] = qt;
 			}
 			__syncthreads();
 		}
@@ -438,6 +464,27 @@ __device__ __forceinline__ void inner_sweep(SH& sh, R tol, R noise, c2<R>* Qg) {
 			Qg[QT ? p0 * MS + i0 + h : (i0 + h) * MS + p0] = xp[h];
 			Qg[QT ? q0 * MS + i0 + h : (i0 + h) * MS + q0] = xq[h];
 		}
+	} else if (!OWN_PAIRS && warp == 4) {
+		const int j = lane & (NR - 1);
+		__syncthreads();
+#pragma unroll 1
+		for (int r = 0; r < ROUNDS; r++) {
+			const T* m = sh.m(r & 1);
+			T* mn = sh.m((r & 1) ^ 1);
+			if (lane < NR) {
+				const int p = first(j, r), q = second(j, r), opq = FULL ? m_at(p, q) : p * LDM + q;
+				const T st = sh.rst[r & 1][j], e = sh.re[r & 1][j];
+				R a = m[p * (LDM + 1)].x, b = m[q * (LDM + 1)].x;
+				T c = m[opq];
+				if (FULL && p > q) c.y = -c.y;
+				rotated_pair(Rotation<R>{st.x, st.y, e.x, e.y}, a, b, c.x, c.y);
+				if (FULL && p > q) c.y = -c.y;
+				mn[p * (LDM + 1)] = mk<R>(a, 0.0);
+				mn[q * (LDM + 1)] = mk<R>(b, 0.0);
+				mn[opq] = c;
+			}
+			__syncthreads();
+		}
 	} else {
 		__syncthreads();
 #pragma unroll 1
@@ -449,8 +496,8 @@ __device__ __forceinline__ void inner_sweep(SH& sh, R tol, R noise, c2<R>* Qg) {
 // Position of player p in round r of the circle method (inverse of rr_player).
 __device__ __forceinline__ int rr_position(int p, int r, int npos) {
 	if (p == 0) return 0;
-	const int m = npos - 1;
-	return ((p - 1 - r) % m + m) % m + 1;
+	const int v = p - 1 - r;  // 0 <= r < npos - 1
+	return v < 0 ? v + npos : v + 1;
 }
 
 // Phase 2 item w of a round: an off-diagonal pair block (jr, jc) of A above the

@@ -10,10 +10,11 @@
 // Before, the sweeps kept all of M and Q in shared memory with two barriers
 // per full round, every block of A was formed (not the upper triangle only),
 // and an item's loads and products came one after the other; whole solves then
-// and now: 3.54 and 2.63 ms at k = 500 (7 sweeps), 17.0 and 11.3 ms at k = 1000
-// (8), 120 and 73 ms at k = 2000 (9). At k = 500 a round is 12 us: 2.5 forming
-// the subproblem, 6.2 in its sweep (760 cycles per inner round, the rotation and
-// the update of M about as long as each other) and 1.3 in the grid barrier.
+// and now: 1.93 and 1.35 ms at k = 256 (8 sweeps), 3.54 and 2.48 ms at k = 500
+// (7), 17.0 and 10.4 ms at k = 1000 (8), 120 and 69 ms at k = 2000 (9). At k =
+// 500 a round is 11.4 us: about 2 forming the subproblem, 6 in its sweep (the
+// rotations and the update of M about as long as each other) and 1.3 in the grid
+// barrier.
 //
 // Accuracy: rotations are unitary to a few FP32 units, so the eigenvector
 // matrix is orthonormal to about 1e-6; normalize_columns_kernel (jacobi.cu)
@@ -120,10 +121,9 @@ __device__ __forceinline__ void group_sync(int g) {
 
 // Phase 1 for pair j of round t (bjacobi.cu phase1_item in FP32; Q is kept as
 // Q(i, l) at [i * MS + l] here).
-__device__ void phase1_item32(Shared32& sh, int j, long long t, int rounds, int nb, int np, int kp,
+__device__ void phase1_item32(Shared32& sh, int j, long long t, int rr, int rounds, int nb, int np, int kp,
 		const float2* prev, const float2* prev2, const float2* Qprev, float2* Qout, float2* out) {
 	const int tid = threadIdx.x;
-	const int rr = (int)(t % rounds);
 	const int P = rr_player(j, rr, nb), Q = rr_player(nb - 1 - j, rr, nb);
 	float2* M = sh.m(0);
 	if (t == 0) {
@@ -132,7 +132,7 @@ __device__ void phase1_item32(Shared32& sh, int j, long long t, int rounds, int 
 			M[i * LDM + l] = __ldcg(prev + (long long)gidx(i, P, Q) * kp + gidx(l, P, Q));
 		}
 	} else {
-		const int ro = (int)((t - 1) % rounds);
+		const int ro = rr ? rr - 1 : rounds - 1;
 		const int posP = rr_position(P, ro, nb), posQ = rr_position(Q, ro, nb);
 		const int a = posP < np ? posP : nb - 1 - posP, hP = posP < np ? 0 : 1;
 		const int b = posQ < np ? posQ : nb - 1 - posQ, hQ = posQ < np ? 0 : 1;
@@ -338,27 +338,29 @@ __global__ void __launch_bounds__(kThreads, 1) bjacobi32_kernel(float2* A0, floa
 	__syncthreads();
 	int sweep = 0;
 	bool stop = false, converged = false;
+	// round t, t mod 3 and t mod rounds (64-bit remainders cost 1000 cycles a round)
 	long long t = 0;
+	int t3 = 0, rr = 0;
 	for (;;) {
 		const bool do_p1 = !stop;
 		// round t + 1's item counter (its last use, round t - 3, is complete)
 		if (blockIdx.x == 0 && tid == 0) p2ctr[(t + 1) & 3] = 0;
 		const bool do_p2 = t >= 1;
 		if (do_p1 && (int)blockIdx.x < p1) {
-			const float2* prev = bufs[t % 3];
-			const float2* prev2 = bufs[(t + 2) % 3];
-			float2* out = bufs[(t + 1) % 3];
+			const float2* prev = bufs[t3];
+			const float2* prev2 = bufs[t3 == 0 ? 2 : t3 - 1];
+			float2* out = bufs[t3 == 2 ? 0 : t3 + 1];
 			for (int j = blockIdx.x; j < np; j += p1)
-				phase1_item32(sh, j, t, rounds, nb, np, kp, prev, prev2, Qbuf + ((t + 1) & 1) * qstride,
+				phase1_item32(sh, j, t, rr, rounds, nb, np, kp, prev, prev2, Qbuf + ((t + 1) & 1) * qstride,
 						Qbuf + (t & 1) * qstride, out);
 		}
 		if (do_p2 && ((int)blockIdx.x >= p2first || join)) {
-			const int ro = (int)((t - 1) % rounds);
-			const float2* src = bufs[(t + 2) % 3];
-			float2* dst = bufs[t % 3];
+			const int ro = rr ? rr - 1 : rounds - 1;
+			const float2* src = bufs[t3 == 0 ? 2 : t3 - 1];
+			float2* dst = bufs[t3];
 			phase2_32(sh, ro, nb, np, nW, kp, src, dst, V, Qbuf + ((t + 1) & 1) * qstride, p2ctr + ((t - 1) & 3));
 		}
-		const bool sweep_end = do_p1 && (t % rounds == rounds - 1);
+		const bool sweep_end = do_p1 && rr == rounds - 1;
 		if (sweep_end && tid == 0) {
 			if (sh.cnt) atomicAdd(&counters[sweep], sh.cnt);
 			if (sh.tmax) atomicMax(&tmaxg[sweep], sh.tmax);
@@ -378,6 +380,8 @@ __global__ void __launch_bounds__(kThreads, 1) bjacobi32_kernel(float2* A0, floa
 			if (sweep >= max_sweeps) stop = true;
 		}
 		t++;
+		t3 = t3 == 2 ? 0 : t3 + 1;
+		rr = rr == rounds - 1 ? 0 : rr + 1;
 	}
 	if (blockIdx.x == 0 && tid == 0) {
 		counters[max_sweeps] = converged ? sweep : -1;
