@@ -220,7 +220,8 @@ bool small_step(const SmallStepArgs& a, int n, int k, cudaStream_t s) {
 			if (sm > 227 * 1024 || !small_pays<G>(a.m, k)) return;
 			const int nc = a.m / 2 + 1;
 			auto kernel = small_step_kernel<R, G::A, G::B>;
-			opt_in_smem(kernel, sm);
+			// on each launch: the limit belongs to the device that is current
+			if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm) != cudaSuccess) return;
 			cudaLaunchAttribute at[1];
 			at[0].id = cudaLaunchAttributeClusterDimension;
 			at[0].val.clusterDim.x = nc;
