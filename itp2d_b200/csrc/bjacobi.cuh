@@ -47,18 +47,30 @@ __device__ __forceinline__ double rsqrt_nr(double x) {
 	return y;
 }
 
-// sin, tau = tan(angle / 2), e and tan of a rotation in double precision
-// throughout, for pairs whose exponents leave the range of the single-precision
-// set-up below: with u = |d| + r and w = 2 r u, cos = u / sqrt(w), |sin| =
-// |c| / sqrt(w) and |tau| = |c| / (sqrt(w) + u), d and c scaled by exact powers
-// of two.
-static __device__ __noinline__ void rotation_wide(double d, double cr, double ci, double& s, double& tau, double& er,
-		double& ei, double& t) {
+// A rotation in double precision throughout, for pairs whose exponents leave
+// the range of the set-up below: with u = |d| + r and w = 2 r u, cos = u / sqrt(w),
+// |sin| = |c| / sqrt(w) and |tau| = |c| / (sqrt(w) + u), d and c scaled by exact
+// powers of two (scalbn: the power itself may leave the range where the values
+// are subnormal). t: the tangent, 0 where |c| / sqrt(|a b|) is at most tol;
+// counted: whether it is above noise.
+struct WideRotation {
+	double s, tau, er, ei, t;
+	bool counted;
+};
+static __device__ __noinline__ WideRotation rotation_wide(double a, double b, double cr, double ci, double tol,
+		double noise) {
+	WideRotation w;
+	// the sizes without products of two elements
+	const double c = hypot(cr, ci);
+	const double scale = sqrt(fabs(a)) * sqrt(fabs(b));
+	w.counted = c > noise * scale;
+	w.s = w.tau = w.er = w.ei = w.t = 0.0;
+	if (!(c > tol * scale)) return w;
+	const double d = 0.5 * (b - a);
 	const double ad = fabs(d);
 	const double mc = fmax(fabs(cr), fabs(ci));
 	const int ex = ilogb(fmax(ad, mc)), exc = ilogb(mc);
-	const double sc = scalbn(1.0, -ex), scc = scalbn(1.0, -exc);
-	const double dn = ad * sc, crn = cr * sc, cin = ci * sc;
+	const double dn = scalbn(ad, -ex), crn = scalbn(cr, -ex), cin = scalbn(ci, -ex);
 	const double cn2 = crn * crn + cin * cin;
 	const double rn2 = dn * dn + cn2;         // [1, 12)
 	const double rn = rn2 * rsqrt_nr(rn2);
@@ -66,14 +78,15 @@ static __device__ __noinline__ void rotation_wide(double d, double cr, double ci
 	const double wn = 2.0 * rn * un;          // [2, 38)
 	const double qn = rsqrt_nr(wn);
 	const double cn = sqrt(cn2);
-	t = cn * rcp_nr(un);
-	const double crs = cr * scc, cis = ci * scc;
+	w.t = cn * rcp_nr(un);
+	const double crs = scalbn(cr, -exc), cis = scalbn(ci, -exc);
 	const double ec = rsqrt_nr(crs * crs + cis * cis);
 	const double sg = d < 0 ? -1.0 : 1.0;
-	s = sg * cn * qn;
-	tau = sg * cn * rcp_nr(wn * qn + un);
-	er = crs * ec;
-	ei = cis * ec;
+	w.s = sg * cn * qn;
+	w.tau = sg * cn * rcp_nr(wn * qn + un);
+	w.er = crs * ec;
+	w.ei = cis * ec;
+	return w;
 }
 
 __device__ __forceinline__ float rsqrt_approx(float x) {
@@ -85,6 +98,15 @@ __device__ __forceinline__ float rcp_approx(float x) {
 	float y;
 	asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
 	return y;
+}
+
+// Whether v >= 0 is between 2^-830 and 2^996 (single precision: 2^-73 and 2^122),
+// by its exponent: squares of tol and noise times v stay normal numbers.
+__device__ __forceinline__ bool well_inside(double v) {
+	return (unsigned)__double2hiint(v) - 0x0C100000u < 0x7E300000u - 0x0C100000u;
+}
+__device__ __forceinline__ bool well_inside(float v) {
+	return __float_as_uint(v) - 0x1B000000u < 0x7C800000u - 0x1B000000u;
 }
 
 // A rotation J = [[cos, s e], [-s conj(e), cos]], cos = 1 - s tau; s = tau = 0
@@ -112,7 +134,8 @@ __device__ __forceinline__ Rotation<R> make_rotation(R a, R b, R cr, R ci, R tol
 	const R scale2 = fabs(a) * fabs(b);
 	const R d = (R)0.5 * (b - a);
 	const R mc = fmax(fabs(cr), fabs(ci));
-	const bool want = c2 > (R)0 && c2 > tol * tol * scale2;
+	bool want = c2 > tol * tol * scale2;
+	bool counted = c2 > noise * noise * scale2;
 	// squares and quotients of d and c stay inside the single-precision range
 	const bool narrow = mc > (R)1e-18 && mc < (R)1e18 && fabs(d) < (R)1e18;
 	const float x = (float)cr, y = (float)ci;
@@ -141,19 +164,22 @@ __device__ __forceinline__ Rotation<R> make_rotation(R a, R b, R cr, R ci, R tol
 	J.s = (R)2 * J.tau * inv;
 	J.er = e0 * f;
 	J.ei = e1 * f;
-	if (want && !narrow) {
-		double s8, tau8, er8, ei8, t8;
-		rotation_wide(d, cr, ci, s8, tau8, er8, ei8, t8);
-		J.s = (R)s8;
-		J.tau = (R)tau8;
-		J.er = (R)er8;
-		J.ei = (R)ei8;
-		t = (R)t8;
+	// the squares decide where |a b| is well inside the range of R (an element
+	// whose square vanishes there is below the threshold)
+	if (mc > (R)0 && (!well_inside(scale2) || (want && !narrow))) {
+		const WideRotation w = rotation_wide(a, b, cr, ci, tol, noise);
+		J.s = (R)w.s;
+		J.tau = (R)w.tau;
+		J.er = (R)w.er;
+		J.ei = (R)w.ei;
+		t = (R)w.t;
+		want = true;
+		counted = w.counted;
 	}
 	if (!want || t == (R)0) {
 		J.s = J.tau = J.ei = (R)0;
 		J.er = (R)1;
-	} else if (c2 > noise * noise * scale2) {
+	} else if (counted) {
 		cnt++;
 		tmax = fmax(tmax, t);
 	}
