@@ -32,6 +32,7 @@ namespace itp2d {
 namespace lines {
 
 constexpr int kSmallThreads = 512;
+constexpr int kSmemMax = 227 * 1024;  // dynamic shared memory a CTA can have
 
 // f(i) for the items i of this thread.
 template <int ITEMS, class F>
@@ -215,13 +216,14 @@ bool small_step(const SmallStepArgs& a, int n, int k, cudaStream_t s) {
 	bool done = false;
 	for_length<R>(n, [&](auto g) {
 		using G = decltype(g);
-		if constexpr (small_smem<G>(1) <= 227 * 1024) {
+		if constexpr (small_smem<G>(1) <= kSmemMax) {
 			const size_t sm = small_smem<G>(a.m);
-			if (sm > 227 * 1024 || !small_pays<G>(a.m, k)) return;
+			if (sm > kSmemMax || !small_pays<G>(a.m, k)) return;
 			const int nc = a.m / 2 + 1;
 			auto kernel = small_step_kernel<R, G::A, G::B>;
-			// on each launch: the limit belongs to the device that is current
-			if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm) != cudaSuccess) return;
+			// on each launch: the limit belongs to the device that is current. It is
+			// the same for every m, since host threads with other m share the kernel
+			cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMax);
 			cudaLaunchAttribute at[1];
 			at[0].id = cudaLaunchAttributeClusterDimension;
 			at[0].val.clusterDim.x = nc;
@@ -234,8 +236,9 @@ bool small_step(const SmallStepArgs& a, int n, int k, cudaStream_t s) {
 			cfg.stream = s;
 			cfg.attrs = at;
 			cfg.numAttrs = 1;
-			cudaLaunchKernelEx(&cfg, kernel, a);
-			done = true;
+			if (e == cudaSuccess) e = cudaLaunchKernelEx(&cfg, kernel, a);
+			done = e == cudaSuccess;
+			if (!done) cudaGetLastError();  // refused: the passes run instead, and report what they meet
 		}
 	});
 	return done;
