@@ -20,6 +20,7 @@
 // (W[i * k + n]: coefficient of state i in output state n).
 #include "../../include/itp2d_gpu.h"
 #include "contract.cuh"
+#include "launch.cuh"
 
 #include <algorithm>
 
@@ -237,21 +238,10 @@ cudaError_t launch_batched_eigensolve(const BatchEigItem* items, int n, int max_
 	const size_t one = kp * kp * sizeof(double2);
 	const size_t cap = 200 * 1024;
 	const int smem = (int)(want <= cap ? want : (one <= cap ? one : 0));
-	if (smem > 48 * 1024) {
-		const cudaError_t e = cudaFuncSetAttribute(batched_jacobi_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-				smem);
-		if (e != cudaSuccess) return e;
-	}
-	static int sms = 0;
-	if (!sms) {
-		int dev = 0;
-		cudaGetDevice(&dev);
-		cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-	}
-	int per_sm = 0;
-	cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, batched_jacobi_kernel, kBThreads, smem);
-	const int grid = std::max(1, std::min(n, std::max(1, per_sm) * std::max(1, sms)));
-	cudaError_t e = cudaMemsetAsync(next, 0, sizeof(int), s);
+	cudaError_t e = raise_smem_limit((const void*)batched_jacobi_kernel, (int)cap);
+	if (e != cudaSuccess) return e;
+	const int grid = std::max(1, std::min(n, resident_ctas((const void*)batched_jacobi_kernel, kBThreads, smem) * sm_count()));
+	e = cudaMemsetAsync(next, 0, sizeof(int), s);
 	if (e != cudaSuccess) return e;
 	batched_jacobi_kernel<<<grid, kBThreads, smem, s>>>(items, n, max_sweeps, smem, next);
 	return cudaGetLastError();

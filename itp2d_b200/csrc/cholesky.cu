@@ -22,6 +22,7 @@
 // counterpart: the reference orthonormalises canonically (stateset.cpp:136-232).
 #include "../../include/itp2d_gpu.h"
 #include "contract.cuh"
+#include "launch.cuh"
 
 #include <algorithm>
 
@@ -299,13 +300,8 @@ size_t cholesky_update_smem() { return sizeof(double2) * (TU * (NB + 1) + NB * (
 
 int launch_cholesky_w(const double2* S, int k, double2* A, double2* X, double2* Linv, double2* W, EigStatus* st,
 		cudaStream_t s) {
-	static bool attr = false;
-	if (!attr) {
-		if (cudaFuncSetAttribute(chol_update_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-				    (int)cholesky_update_smem()) != cudaSuccess)
-			return ITP2D_E_CUDA;
-		attr = true;
-	}
+	if (raise_smem_limit((const void*)chol_update_kernel, (int)cholesky_update_smem()) != cudaSuccess)
+		return ITP2D_E_CUDA;
 	cudaError_t e = cudaMemsetAsync(st, 0, sizeof(EigStatus), s);
 	if (e == cudaSuccess) e = cudaMemcpyAsync(A, S, (size_t)k * k * sizeof(double2), cudaMemcpyDeviceToDevice, s);
 	if (e != cudaSuccess) return ITP2D_E_CUDA;

@@ -14,6 +14,7 @@
 #include <mutex>
 
 #include "contract.cuh"
+#include "launch.cuh"
 #include "../../include/itp2d_gpu.h"
 
 namespace itp2d {
@@ -253,7 +254,8 @@ cudaError_t launch_eigh(double2* S, int k, JacobiWork& w, EigStatus* st, int num
 	int P = 1;
 	while (P < k) P <<= 1;
 	const size_t smem = (size_t)P * (sizeof(double) + sizeof(int));
-	if (smem > 48 * 1024) cudaFuncSetAttribute(eig_sort_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+	// up to 16384 keys (the kernel has static shared memory beside them)
+	if (smem > 48 * 1024) raise_smem_limit((const void*)eig_sort_kernel, 192 * 1024);
 	eig_sort_kernel<<<1, 1024, smem, s>>>(w.A0, w.A1, w.A2, k, kp, w.counters, w.max_sweeps, w.evals, w.perm,
 			st, check);
 	return cudaGetLastError();

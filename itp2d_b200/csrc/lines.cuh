@@ -22,13 +22,10 @@
 // RowPassArgs / ColPassArgs.
 #pragma once
 
+#include "launch.cuh"
 #include "split.cuh"
 
 #include <algorithm>
-#include <map>
-#include <mutex>
-#include <set>
-#include <tuple>
 #include <type_traits>
 #include <utility>
 
@@ -883,47 +880,12 @@ __global__ void __launch_bounds__((Geo<R, A, B>::COL_THREADS), (Geo<R, A, B>::EN
 	}
 }
 
-template <class K>
-void opt_in_smem(K kernel, size_t bytes) {
-	static std::mutex mu;
-	static std::set<const void*> done;
-	std::lock_guard<std::mutex> g(mu);
-	if (bytes > 48 * 1024 && done.insert((const void*)kernel).second)
-		cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
-}
-
-inline int sm_count() {
-	static int sms = [] {
-		int dev = 0, n = 0;
-		cudaGetDevice(&dev);
-		cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
-		return n > 0 ? n : 1;
-	}();
-	return sms;
-}
-
-// Persistent grid: as many CTAs as fit on the device, at most one per tile. The
-// occupancy of a kernel at a launch shape is asked for once (the query costs as
-// much host time as a launch; a solve of 48 states on 96 x 96: 28.6 -> 27.5 ms).
+// Persistent grid: as many CTAs as fit on the device, at most one per tile.
 template <class K>
 int grid_for(K kernel, int threads, size_t smem, long long tiles) {
-	static std::mutex mu;
-	static std::map<std::tuple<const void*, int, size_t>, int> known;
-	int per_sm = 0;
-	{
-		std::lock_guard<std::mutex> g(mu);
-		const auto key = std::make_tuple((const void*)kernel, threads, smem);
-		const auto it = known.find(key);
-		if (it != known.end()) {
-			per_sm = it->second;
-		} else {
-			opt_in_smem(kernel, smem);
-			cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, smem);
-			per_sm = std::max(1, per_sm);
-			known.emplace(key, per_sm);
-		}
-	}
-	return (int)std::max(1LL, std::min((long long)per_sm * sm_count(), tiles));
+	if (smem > 48 * 1024) raise_smem_limit((const void*)kernel);
+	const long long resident = resident_ctas((const void*)kernel, threads, smem);
+	return (int)std::max(1LL, std::min(resident * sm_count(), tiles));
 }
 
 // Rows per tile: a full CTA's worth, fewer where that leaves the device

@@ -32,7 +32,6 @@ namespace itp2d {
 namespace lines {
 
 constexpr int kSmallThreads = 512;
-constexpr int kSmemMax = 227 * 1024;  // dynamic shared memory a CTA can have
 
 // f(i) for the items i of this thread.
 template <int ITEMS, class F>
@@ -221,9 +220,7 @@ bool small_step(const SmallStepArgs& a, int n, int k, cudaStream_t s) {
 			if (sm > kSmemMax || !small_pays<G>(a.m, k)) return;
 			const int nc = a.m / 2 + 1;
 			auto kernel = small_step_kernel<R, G::A, G::B>;
-			// on each launch: the limit belongs to the device that is current. It is
-			// the same for every m, since host threads with other m share the kernel
-			cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMax);
+			cudaError_t e = raise_smem_limit((const void*)kernel);
 			cudaLaunchAttribute at[1];
 			at[0].id = cudaLaunchAttributeClusterDimension;
 			at[0].val.clusterDim.x = nc;

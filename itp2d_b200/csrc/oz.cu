@@ -37,6 +37,7 @@
 
 #include "../../include/itp2d_gpu.h"
 #include "contract.cuh"
+#include "launch.cuh"
 #include "tcgen05.cuh"
 
 namespace itp2d {
@@ -595,12 +596,8 @@ size_t oz_exp_ints(int k, long long G) {
 }
 
 static void oz_attributes() {
-	static bool attr = false;
-	if (!attr) {
-		cudaFuncSetAttribute(rotate_oz_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)oz_smem());
-		cudaFuncSetAttribute(overlap_oz_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)oz_smem());
-		attr = true;
-	}
+	raise_smem_limit((const void*)rotate_oz_kernel, (int)oz_smem());
+	raise_smem_limit((const void*)overlap_oz_kernel, (int)oz_smem());
 }
 
 void launch_rotate_oz(const double2* W, const double2* psi, int k, long long G, unsigned char* wsl,

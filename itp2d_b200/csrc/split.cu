@@ -6,11 +6,10 @@
 // is (k states, tiles) with the state index fastest so that CTAs running at the
 // same time read the same rows of the (state-independent) tables from L2.
 #include "fft.cuh"
+#include "launch.cuh"
 #include "split.cuh"
 
 #include <algorithm>
-#include <mutex>
-#include <set>
 
 namespace itp2d {
 
@@ -494,17 +493,6 @@ __global__ void energy_finish_kernel(const double* __restrict__ sums, const doub
 	}
 }
 
-// Opts a kernel into the full 227 KB of dynamic shared memory once per
-// kernel (keyed by its address: float and double instantiations share a type).
-template <class K>
-void set_smem_limit(K kernel) {
-	static std::mutex mu;
-	static std::set<const void*> done;
-	std::lock_guard<std::mutex> g(mu);
-	if (done.insert((const void*)kernel).second)
-		cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
-}
-
 }  // namespace
 
 int row_tile_rows(int L, int elem_bytes, int sy) {
@@ -534,15 +522,7 @@ size_t col_pass_smem(int L, int cols, int n_fft, int elem_bytes) {
 // Persistent grid: as many CTAs as fit on the device, at most one per tile.
 template <class K>
 int persistent_blocks(K kernel, size_t smem, long long tiles) {
-	static int sms = 0;
-	if (!sms) {
-		int dev = 0;
-		cudaGetDevice(&dev);
-		cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-	}
-	int per_sm = 0;
-	cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kThreads, smem);
-	const long long b = (long long)std::max(1, per_sm) * std::max(1, sms);
+	const long long b = (long long)resident_ctas((const void*)kernel, kThreads, smem) * sm_count();
 	return (int)std::max(1LL, std::min(b, tiles));
 }
 
@@ -557,7 +537,7 @@ template <class R>
 void launch_dm_row_pass(const DmRowArgs& a, int k, cudaStream_t s) {
 	const size_t es = sizeof(c2<R>);
 	const size_t sm = (size_t)4 * a.rows_per_tile * 2 * a.sx * es + (size_t)a.lp_dst.fft.n * es;
-	set_smem_limit(dm_row_kernel<R>);
+	raise_smem_limit((const void*)dm_row_kernel<R>);
 	const dim3 grid(k, (a.sy + a.rows_per_tile - 1) / a.rows_per_tile);
 	dm_row_kernel<R><<<grid, kThreads, sm, s>>>(a);
 }
@@ -567,7 +547,7 @@ void launch_row_pass(const RowPassArgs& a, int k, const void*, cudaStream_t s) {
 	if (launch_row_pass_reg<R>(a, k, s) || launch_row_pass_sine<R>(a, k, s)) return;
 	const int L = a.lp.kind == 0 ? a.sx : 2 * a.sx;
 	const size_t sm = pipe_smem(L, a.rows_per_tile, a.lp.fft.n, sizeof(c2<R>));
-	set_smem_limit(row_pass_kernel<R>);
+	raise_smem_limit((const void*)row_pass_kernel<R>);
 	const long long tiles = (long long)k * ((a.sy + a.rows_per_tile - 1) / a.rows_per_tile);
 	row_pass_kernel<R><<<persistent_blocks(row_pass_kernel<R>, sm, tiles), kThreads, sm, s>>>(a, k);
 }
@@ -577,7 +557,7 @@ void launch_col_pass(const ColPassArgs& a, int k, const void*, cudaStream_t s) {
 	if (launch_col_pass_reg<R>(a, k, s) || launch_col_pass_sine<R>(a, k, s)) return;
 	const int L = a.lp.kind == 0 ? a.sy : 2 * a.sy;
 	const size_t sm = pipe_smem(L, a.cols_per_tile, a.lp.fft.n, sizeof(c2<R>));
-	set_smem_limit(col_pass_kernel<R>);
+	raise_smem_limit((const void*)col_pass_kernel<R>);
 	const long long tiles = (long long)k * ((a.sx + a.cols_per_tile - 1) / a.cols_per_tile);
 	col_pass_kernel<R><<<persistent_blocks(col_pass_kernel<R>, sm, tiles), kThreads, sm, s>>>(a, k);
 }
@@ -588,7 +568,7 @@ void launch_energy_row(const EnergyRowArgs& a, int k, const void*, cudaStream_t 
 	const int L = a.lp.kind == 0 ? a.sx : 2 * a.sx;
 	const dim3 grid(k, (a.sy + a.rows_per_tile - 1) / a.rows_per_tile);
 	const size_t sm = row_pass_smem(L, a.rows_per_tile, a.lp.fft.n, sizeof(c2<R>));
-	set_smem_limit(energy_row_kernel<R>);
+	raise_smem_limit((const void*)energy_row_kernel<R>);
 	energy_row_kernel<R><<<grid, kThreads, sm, s>>>(a);
 }
 
@@ -598,7 +578,7 @@ void launch_energy_col(const EnergyColArgs& a, int k, const void*, cudaStream_t 
 	const int L = a.lp.kind == 0 ? a.sy : 2 * a.sy;
 	const dim3 grid(k, (a.sx + a.cols_per_tile - 1) / a.cols_per_tile);
 	const size_t sm = col_pass_smem(L, a.cols_per_tile, a.lp.fft.n, sizeof(c2<R>));
-	set_smem_limit(energy_col_kernel<R>);
+	raise_smem_limit((const void*)energy_col_kernel<R>);
 	energy_col_kernel<R><<<grid, kThreads, sm, s>>>(a);
 }
 
