@@ -416,13 +416,85 @@ __global__ void __launch_bounds__(kThreads, 1) bjacobi_kernel(double2* A0, doubl
 	}
 }
 
+// The whole solve of a matrix of at most kTinyN indices by one warp, pair after
+// pair (lane i: element i of the two rows and columns that a rotation touches). A
+// sweep is 1 to 6 rotations in line here and 31 rounds of 1000 cycles in the
+// block kernel, whatever n; beyond four the block kernel's round of 16 rotations
+// wins. Allocation-free eigensolve, n = 1, 2, 3, 4: block kernel 101, 139, 169,
+// 188 us, this one 74, 74, 79,
+// 85. A kernel of its own: the same sweep as a branch of
+// bjacobi_kernel cost that kernel 7 % of its time at k = 200.
+constexpr int kTinyN = 4;
+__global__ void __launch_bounds__(32) tiny_jacobi_kernel(double2* A, double2* V, int n, int kp, int max_sweeps,
+		double tol, double tau_final, int* counters) {
+	__shared__ double2 M[kTinyN * LDM], Q[kTinyN][kTinyN];  // upper triangle; Q(i, l) at [l][i]
+	const int i = threadIdx.x;
+	for (int e = i; e < n * n; e += 32) {
+		const int r = e / n, l = e % n;
+		if (r <= l) M[m_at(r, l)] = A[(long long)r * kp + l];
+		Q[l][r] = make_double2(r == l ? 1.0 : 0.0, 0.0);
+	}
+	__syncwarp();
+	int sweep = 0;
+	bool converged = false;
+	while (!converged && sweep < max_sweeps) {
+		int cnt = 0;
+		double tmax = 0.0;
+#pragma unroll 1
+		for (int p = 0; p + 1 < n; p++)
+#pragma unroll 1
+			for (int q = p + 1; q < n; q++) {
+				double a = M[m_at(p, p)].x, b = M[m_at(q, q)].x;
+				double2 c = M[m_at(p, q)];
+				const Rotation<double> J = make_rotation<double>(a, b, c.x, c.y, tol, kNoiseRel, cnt, tmax);
+				rotated_pair(J, a, b, c.x, c.y);
+				__syncwarp();
+				if (i < n) {
+					if (i != p && i != q) {
+						double2 xp = ld_m(M, p, i), xq = ld_m(M, q, i);
+						rows2(J.s, J.tau, J.er, J.ei, xp.x, xp.y, xq.x, xq.y);
+						st_m(M, p, i, xp);
+						st_m(M, q, i, xq);
+					}
+					if (i == p) {
+						M[m_at(p, p)] = make_double2(a, 0.0);
+						M[m_at(q, q)] = make_double2(b, 0.0);
+						M[m_at(p, q)] = c;
+					}
+					double2 vp = Q[p][i], vq = Q[q][i];
+					cols2(J.s, J.tau, J.er, J.ei, vp.x, vp.y, vq.x, vq.y);
+					Q[p][i] = vp;
+					Q[q][i] = vq;
+				}
+				__syncwarp();
+			}
+		sweep++;
+		converged = cnt == 0 || tmax < tau_final;  // the same in every lane
+	}
+	for (int e = i; e < n * n; e += 32) {
+		const int r = e / n, l = e % n;
+		A[(long long)r * kp + l] = ld_m(M, r, l);
+		V[(long long)r * kp + l] = Q[l][r];
+	}
+	if (i == 0) {
+		counters[max_sweeps] = converged ? sweep : -1;
+		counters[max_sweeps + 1] = 0;
+	}
+}
+
 }  // namespace
 
 int bjacobi_padded(int k) { return ((k + MS - 1) / MS) * MS; }
 size_t bjacobi_qbuf_elems(int k) { return 2 * (size_t)(bjacobi_padded(k) / MS) * MS * MS; }
 
-cudaError_t launch_bjacobi(double2* A0, double2* A1, double2* A2, double2* V, double2* Qbuf, int kp,
+cudaError_t launch_bjacobi(double2* A0, double2* A1, double2* A2, double2* V, double2* Qbuf, int n, int kp,
 		int max_sweeps, double tau_final, int* counters, int num_sms, cudaStream_t s) {
+	double tol = 1e-15;
+	if (!(tau_final > 0.0)) tau_final = kTauFinal;
+	if (n <= kTinyN) {
+		tiny_jacobi_kernel<<<1, 32, 0, s>>>(A0, V, n, kp, max_sweeps, tol, tau_final, counters);
+		return cudaGetLastError();
+	}
 	const size_t smem = sizeof(Shared);
 	cudaError_t e = cudaFuncSetAttribute(bjacobi_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
 	if (e != cudaSuccess) return e;
@@ -434,8 +506,6 @@ cudaError_t launch_bjacobi(double2* A0, double2* A1, double2* A2, double2* V, do
 	// the grid barrier of a small problem spans few CTAs
 	const int np = kp / MS, nW = np * (np - 1) / 2 + np * np;
 	const int blocks = std::min(num_sms, np + (nW + 1) / 2);
-	double tol = 1e-15;
-	if (!(tau_final > 0.0)) tau_final = kTauFinal;
 	unsigned long long* tmax = reinterpret_cast<unsigned long long*>(counters + jacobi_tmax_offset(max_sweeps));
 	int* p2ctr = counters + jacobi_p2ctr_offset(max_sweeps);
 	void* args[] = {&A0, &A1, &A2, &V, &Qbuf, &kp, &max_sweeps, &tol, &tau_final, &counters, &tmax, &p2ctr};

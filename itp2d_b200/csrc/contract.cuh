@@ -97,7 +97,7 @@ int bjacobi_padded(int k);
 size_t bjacobi_qbuf_elems(int k);
 // Row stride of the eigensolver's matrices: A0, A1, A2 and V are kp x kp.
 int jacobi_kp(int k);
-cudaError_t launch_bjacobi(double2* A0, double2* A1, double2* A2, double2* V, double2* Qbuf, int kp,
+cudaError_t launch_bjacobi(double2* A0, double2* A1, double2* A2, double2* V, double2* Qbuf, int n, int kp,
 		int max_sweeps, double tau_final, int* counters, int num_sms, cudaStream_t s);
 // Single-precision block Jacobi of S (k x k, FP64) on w.f32; leaves the
 // eigenvalues on the diagonal of w.A0, the eigenvectors in w.V and the result

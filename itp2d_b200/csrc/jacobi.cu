@@ -242,7 +242,7 @@ cudaError_t launch_eigh(double2* S, int k, JacobiWork& w, EigStatus* st, int num
 	} else {
 		jacobi_init_kernel<<<(unsigned)std::min<long long>((n + 255) / 256, 4096), 256, 0, s>>>(S, k, kp, w.A0,
 				w.V);
-		e = launch_bjacobi(w.A0, w.A1, w.A2, w.V, w.Qbuf, kp, w.max_sweeps, w.tau_final, w.counters, num_sms, s);
+		e = launch_bjacobi(w.A0, w.A1, w.A2, w.V, w.Qbuf, k, kp, w.max_sweeps, w.tau_final, w.counters, num_sms, s);
 	}
 	if (e != cudaSuccess) return e;
 	if (serial.owns_lock()) {
