@@ -419,10 +419,10 @@ __global__ void __launch_bounds__(kThreads, 1) bjacobi_kernel(double2* A0, doubl
 // The whole solve of a matrix of at most kTinyN indices by one warp, pair after
 // pair (lane i: element i of the two rows and columns that a rotation touches). A
 // sweep is 1 to 6 rotations in line here and 31 rounds of 1000 cycles in the
-// block kernel, whatever n; beyond four the block kernel's round of 16 rotations
-// wins. Allocation-free eigensolve, n = 1, 2, 3, 4: block kernel 101, 139, 169,
-// 188 us, this one 74, 74, 79,
-// 85. A kernel of its own: the same sweep as a branch of
+// block kernel, whatever n. Allocation-free eigensolve, n = 1, 2, 3, 4: block
+// kernel 101, 139, 169, 188 us, this one 74, 74, 79, 85 (a cooperative kernel of
+// one grid-wide round per n / 2 rotations: 82, 85, 161, 184, and 266 against the
+// block kernel's 190 at n = 5). A kernel of its own: the same sweep as a branch of
 // bjacobi_kernel cost that kernel 7 % of its time at k = 200.
 constexpr int kTinyN = 4;
 __global__ void __launch_bounds__(32) tiny_jacobi_kernel(double2* A, double2* V, int n, int kp, int max_sweeps,

@@ -297,13 +297,14 @@ KTables ktables(const itp2d_ctx* c) {
 }
 
 // Multi-product coefficients c_t = t^{2(m-1)} / prod_{n != t}(t^2 - n^2)
-// (multiproductsplit.cpp:49-59).
+// (multiproductsplit.cpp:49-59, which multiplies integers). The products pass
+// 2^31 at m = 8 (1.6e11): they are exact in double.
 std::vector<double> mp_coefficients(int m) {
 	std::vector<double> c(m);
 	for (int t = 1; t <= m; t++) {
-		int denom = 1;
+		double denom = 1.0;
 		for (int n = 1; n <= m; n++)
-			if (n != t) denom *= (t * t - n * n);
+			if (n != t) denom *= t * t - n * n;
 		c[t - 1] = std::pow((double)t, 2 * (m - 1)) / denom;
 	}
 	return c;
