@@ -18,16 +18,17 @@ def capi():
     return C
 
 
-# one launch (40 x 40), line passes (40 x 48), sine passes (40 x 48, hard walls)
+# one launch (40 x 40), also with a field, line passes (40 x 48), sine passes (40 x 48, hard walls)
 @pytest.mark.parametrize("precision", ["fp64", "fp32"])
-@pytest.mark.parametrize("sy,boundary", [(40, O.PERIODIC), (48, O.PERIODIC), (48, O.DIRICHLET)])
+@pytest.mark.parametrize("sy,boundary,B", [(40, O.PERIODIC, 0.0), (40, O.PERIODIC, 0.8), (48, O.PERIODIC, 0.0),
+                                           (48, O.DIRICHLET, 0.0)])
 @pytest.mark.parametrize("m", [6, 7, 8])
-def test_step_matches_oracle(capi, m, sy, boundary, precision):
+def test_step_matches_oracle(capi, m, sy, boundary, B, precision):
     g = O.Grid(40, sy, 0.2)
     V = O.harmonic(g)
     psi = O.gaussian_states(g, 3, m)
-    ref = O.MultiProductSplit(g, V, boundary, 0.0, m, 0.05)
-    c = capi.Context(40, sy, g.dx, 3, boundary, 0.0, m, capi.FP64 if precision == "fp64" else capi.FP32)
+    ref = O.MultiProductSplit(g, V, boundary, B, m, 0.05)
+    c = capi.Context(40, sy, g.dx, 3, boundary, B, m, capi.FP64 if precision == "fp64" else capi.FP32)
     c.set_potential(V)
     c.set_time_step(0.05)
     c.upload(psi)
