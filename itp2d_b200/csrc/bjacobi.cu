@@ -289,7 +289,8 @@ __device__ __forceinline__ void phase2_item(double2 (*st)[OP], const Item& it, i
 // during the products of the current one. Bound: DMMA issue and the operands'
 // L2 traffic (48 KB in, 32 KB out per block of A); whole eigensolves, upper
 // triangle and copies ahead against all blocks with loads in line: 21.4 -> 17.7
-// ms at k = 1000 (9 sweeps), 161 -> 124 ms at k = 2000 (10 sweeps).
+// ms at k = 1000 (9 sweeps), 161 -> 124 ms at k = 2000 (10 sweeps); the whole
+// solves take 16.4 and 112 ms with the cheaper indices of the rounds.
 __device__ void phase2(Shared& sh, int ro, int nb, int np, int nW, int kp, const double2* src, double2* dst,
 		double2* V, const double2* Qr, int* ctr) {
 	const int half = threadIdx.x / (kThreads / 2), lt = threadIdx.x & (kThreads / 2 - 1);

@@ -56,7 +56,7 @@ __global__ void chol_identity_kernel(double2* X, int k) {
 // barriers per pivot; the thread of the next pivot prepares its reciprocal
 // square root right after its update. Latency-bound: a chain of 32 pivots
 // (39 us with the inverse substituted afterwards by one thread per column,
-// 20 us now).
+// 18 us now).
 __global__ void __launch_bounds__(1024) chol_diag_kernel(double2* A, int k, int j, double2* Linv, EigStatus* st) {
 	__shared__ double2 lcol[NB], xrow[NB];  // column p of L, row p of X
 	__shared__ double s_pivot[2], s_inv[2];

@@ -327,7 +327,7 @@ int overlap_splits(int k, long long G, int num_sms) {
 	// two CTAs per SM (80 KB of stages each for FP64 states); splits of at
 	// least 128 grid points (8 steps: fewer would not cover the two latencies at
 	// their ends; 512 left 18 CTAs for 48 states on 96 x 96 and took 105 us,
-	// 37 us now), up to enough for two waves (at least 16); the
+	// 35 us now), up to enough for two waves (at least 16); the
 	// first count whose grid fills its last wave to 95 % or more, else the
 	// best-filled one (k = 2000: 528 tile pairs fill 1.78 waves unsplit, 5
 	// splits fill 8.92 waves; a few tile pairs take as many splits as fill

@@ -2,8 +2,8 @@
 //
 // Replaces EigenSolver::solve (ZHEEV, eigensolver.hpp:80-84) and the checks
 // and scaling of StateSet::orthonormalize (stateset.cpp:155-176): the block
-// Jacobi iteration of bjacobi.cu (FP64, every k) or bjacobi32.cu (FP32 states
-// of kBlockJacobi32MinK and more), then the steps of this file: unit columns,
+// Jacobi iteration of bjacobi.cu (FP64, every k; up to 4 in one warp) or
+// bjacobi32.cu (FP32 states of kBlockJacobi32MinK and more), then the steps of this file: unit columns,
 // the ascending sort with the reference's checks, and W = V l^{-1/2}.
 //
 // FP64 block Jacobi serves small k too: a sweep of k = 200 takes 13 grid-wide

@@ -231,28 +231,6 @@ template <> struct Roots<25> {
 		return t[j];
 	}
 };
-template <> struct Roots<30> {
-	static constexpr __host__ __device__ double c(int j) {
-		constexpr double t[30] = {
-				1.0, 0.9781476007338057, 0.9135454576426009, 0.8090169943749475, 0.6691306063588582, 0.5,
-				0.30901699437494745, 0.10452846326765347, -0.10452846326765347, -0.30901699437494745, -0.5,
-				-0.6691306063588582, -0.8090169943749475, -0.9135454576426009, -0.9781476007338057, -1.0,
-				-0.9781476007338057, -0.9135454576426009, -0.8090169943749475, -0.6691306063588582, -0.5,
-				-0.30901699437494745, -0.10452846326765347, 0.10452846326765347, 0.30901699437494745, 0.5,
-				0.6691306063588582, 0.8090169943749475, 0.9135454576426009, 0.9781476007338057};
-		return t[j];
-	}
-	static constexpr __host__ __device__ double s(int j) {
-		constexpr double t[30] = {
-				0.0, 0.20791169081775934, 0.4067366430758002, 0.5877852522924731, 0.7431448254773942, 0.8660254037844386,
-				0.9510565162951535, 0.9945218953682733, 0.9945218953682733, 0.9510565162951535, 0.8660254037844386,
-				0.7431448254773942, 0.5877852522924731, 0.4067366430758002, 0.20791169081775934, 0.0, -0.20791169081775934,
-				-0.4067366430758002, -0.5877852522924731, -0.7431448254773942, -0.8660254037844386, -0.9510565162951535,
-				-0.9945218953682733, -0.9945218953682733, -0.9510565162951535, -0.8660254037844386, -0.7431448254773942,
-				-0.5877852522924731, -0.4067366430758002, -0.20791169081775934};
-		return t[j];
-	}
-};
 template <> struct Roots<32> {
 	static constexpr __host__ __device__ double c(int j) {
 		constexpr double t[32] = {

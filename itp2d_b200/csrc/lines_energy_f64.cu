@@ -3,6 +3,8 @@
 
 namespace itp2d {
 
+// (the FP64 tile for both precisions: an FP32 CTA has at most 128 of the 256
+// threads that its kernel is compiled for)
 int energy_row_tile_reg(const LinePlan& lp, int sy, int k) {
 	int n = 0;
 	if (lp.kind == 0)

@@ -8,11 +8,11 @@
 // longest member alone; then the cluster adds the members out of each other's
 // shared memory in the order of the passes ((m1 + m2) + m3 ...). A member's
 // chain runs on one SM, in stages of 512 threads with a barrier between them: 25
-// states of 64 x 64 (FP64, 10th order) take 37 us on an idle device and 19 us a
-// step where two sets take turns, in place of 93. A stage of 4096 points takes
-// 1900 cycles: 1270 of shared-memory traffic and 700 of FP64 work that the
-// barriers keep from overlapping wholly (tables brought into L1 ahead, or row
-// stages that wait for their warp alone, changed nothing).
+// states of 64 x 64 (FP64, 10th order) take 37 us, in place of 93; two contexts
+// that step in turn, each on its own stream, overlap and take 19 us a step. A
+// stage of 4096 points takes 1900 cycles: 1270 of shared-memory traffic and 700
+// of FP64 work that the barriers keep from overlapping wholly (tables brought into
+// L1 ahead, or row stages that wait for their warp alone, changed nothing).
 //
 // The stages are those of lines.cuh, all in place: an alpha item of row y reads
 // and writes the slots [k1][b] of its b, a beta item those of its k1 (rows of A
