@@ -30,7 +30,8 @@
 // rounding level of the phase-2 products (below 1e-13) do not count against
 // convergence; the iteration stops after a sweep whose largest counted
 // rotation tangent is below tau_final (3e-9 by default: quadratic convergence
-// then leaves off-diagonal elements of order k * 1e-17 relative to the gaps).
+// then leaves off-diagonal elements of order k * 1e-17 relative to the gaps) and
+// in which no rotated element was above 1e-8 of sqrt(|A_pp A_qq|).
 #include <cooperative_groups.h>
 
 #include "../../include/itp2d_gpu.h"

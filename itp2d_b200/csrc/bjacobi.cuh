@@ -52,10 +52,10 @@ __device__ __forceinline__ double rsqrt_nr(double x) {
 // |sin| = |c| / sqrt(w) and |tau| = |c| / (sqrt(w) + u), d and c scaled by exact
 // powers of two (scalbn: the power itself may leave the range where the values
 // are subnormal). t: the tangent, 0 where |c| / sqrt(|a b|) is at most tol;
-// counted: whether it is above noise.
+// counted: whether it is above noise; coarse: whether it is above 2^-26.
 struct WideRotation {
 	double s, tau, er, ei, t;
-	bool counted;
+	bool counted, coarse;
 };
 static __device__ __noinline__ WideRotation rotation_wide(double a, double b, double cr, double ci, double tol,
 		double noise) {
@@ -64,6 +64,7 @@ static __device__ __noinline__ WideRotation rotation_wide(double a, double b, do
 	const double c = hypot(cr, ci);
 	const double scale = sqrt(fabs(a)) * sqrt(fabs(b));
 	w.counted = c > noise * scale;
+	w.coarse = c > 0x1p-26 * scale;
 	w.s = w.tau = w.er = w.ei = w.t = 0.0;
 	if (!(c > tol * scale)) return w;
 	const double d = 0.5 * (b - a);
@@ -109,6 +110,12 @@ __device__ __forceinline__ bool well_inside(float v) {
 	return __float_as_uint(v) - 0x1B000000u < 0x7C800000u - 0x1B000000u;
 }
 
+// Whether c2 / scale2 is above about 2^-52, by exponents (2^-53 to 2^-51).
+__device__ __forceinline__ bool above_half_precision(double c2, double scale2) {
+	return __double2hiint(c2) - __double2hiint(scale2) > -(52 << 20);
+}
+__device__ __forceinline__ bool above_half_precision(float, float) { return false; }
+
 // A rotation J = [[cos, s e], [-s conj(e), cos]], cos = 1 - s tau; s = tau = 0
 // and e = 1 when the pair is not rotated.
 template <class R>
@@ -127,7 +134,12 @@ struct Rotation {
 // In double precision this replaces a chain of five Newton-refined square roots
 // and reciprocals (about 40 dependent operations of 8.5 cycles) by about eight,
 // on the critical path of every inner round. Counted rotations (relative size
-// above `noise`) and the largest counted tangent accumulate in cnt and tmax.
+// above `noise`) and the largest counted tangent accumulate in cnt and tmax. In
+// double precision a rotation of a relative size above 2^-26 counts with a tangent
+// of one: it leaves 1e-7 of its element, which is more than rounding beside
+// sqrt(|a b|), so that its sweep must not be the last. The tangent alone does not
+// say so where the diagonals differ by many decades (1e-9 may go with an element
+// as large as sqrt(|a b|)).
 template <class R>
 __device__ __forceinline__ Rotation<R> make_rotation(R a, R b, R cr, R ci, R tol, R noise, int& cnt, R& tmax) {
 	const R c2 = cr * cr + ci * ci;
@@ -136,6 +148,7 @@ __device__ __forceinline__ Rotation<R> make_rotation(R a, R b, R cr, R ci, R tol
 	const R mc = fmax(fabs(cr), fabs(ci));
 	bool want = c2 > tol * tol * scale2;
 	bool counted = c2 > noise * noise * scale2;
+	bool coarse = above_half_precision(c2, scale2);
 	// squares and quotients of d and c stay inside the single-precision range
 	const bool narrow = mc > (R)1e-18 && mc < (R)1e18 && fabs(d) < (R)1e18;
 	const float x = (float)cr, y = (float)ci;
@@ -175,13 +188,14 @@ __device__ __forceinline__ Rotation<R> make_rotation(R a, R b, R cr, R ci, R tol
 		t = (R)w.t;
 		want = true;
 		counted = w.counted;
+		coarse = sizeof(R) == 8 && w.coarse;
 	}
 	if (!want || t == (R)0) {
 		J.s = J.tau = J.ei = (R)0;
 		J.er = (R)1;
 	} else if (counted) {
 		cnt++;
-		tmax = fmax(tmax, t);
+		tmax = coarse ? (R)1 : fmax(tmax, t);
 	}
 	return J;
 }
