@@ -126,13 +126,16 @@ __device__ __forceinline__ void half_sync(int half) {
 // (upper triangle of M buffer 0), sweeps it, stores Q_t and the rotated
 // subproblem. prev: A_{t-1} (diagonal pair blocks of round t - 1), prev2:
 // A_{t-2}, Qprev: the Q buffer of round t - 1 (t >= 1). For t = 0 the
-// subproblem is read from prev = A_{-1}, the initial matrix.
+// subproblem is read from prev = A_{-1}, the initial matrix, and a matrix of one
+// pair from prev in every round: phase 1 of round t - 1 left all of it there.
+// (Forming its off-diagonal block by products again would put the rounding of the
+// large eigenvalues beside the null ones, whose rotations would then never end.)
 __device__ void phase1_item(Shared& sh, int j, long long t, int rr, int rounds, int nb, int np, int kp, double tol,
 		const double2* prev, const double2* prev2, const double2* Qprev, double2* Qout, double2* out) {
 	const int tid = threadIdx.x;
 	const int P = rr_player(j, rr, nb), Q = rr_player(nb - 1 - j, rr, nb);
 	double2* M = sh.m(0);
-	if (t == 0) {
+	if (t == 0 || np == 1) {
 		for (int e = tid; e < MS * MS; e += kThreads) {
 			const int i = e / MS, l = e % MS;
 			M[i * LDM + l] = __ldcg(prev + (long long)gidx(i, P, Q) * kp + gidx(l, P, Q));
