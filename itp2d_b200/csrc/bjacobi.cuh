@@ -136,10 +136,10 @@ struct Rotation {
 // on the critical path of every inner round. Counted rotations (relative size
 // above `noise`) and the largest counted tangent accumulate in cnt and tmax. In
 // double precision a rotation of a relative size above 2^-26 counts with a tangent
-// of one: it leaves 1e-7 of its element, which is more than rounding beside
-// sqrt(|a b|), so that its sweep must not be the last. The tangent alone does not
-// say so where the diagonals differ by many decades (1e-9 may go with an element
-// as large as sqrt(|a b|)).
+// of at least 2^-28, above the tangent that ends the sweeps by default: it leaves
+// 1e-7 of its element, which is more than rounding beside sqrt(|a b|). The tangent
+// alone does not say so where the diagonals differ by many decades (1e-9 may go
+// with an element as large as sqrt(|a b|)).
 template <class R>
 __device__ __forceinline__ Rotation<R> make_rotation(R a, R b, R cr, R ci, R tol, R noise, int& cnt, R& tmax) {
 	const R c2 = cr * cr + ci * ci;
@@ -195,7 +195,7 @@ __device__ __forceinline__ Rotation<R> make_rotation(R a, R b, R cr, R ci, R tol
 		J.er = (R)1;
 	} else if (counted) {
 		cnt++;
-		tmax = coarse ? (R)1 : fmax(tmax, t);
+		tmax = fmax(tmax, coarse ? fmax(t, (R)0x1p-28) : t);
 	}
 	return J;
 }
