@@ -31,7 +31,12 @@
 // convergence; the iteration stops after a sweep whose largest counted
 // rotation tangent is below tau_final (3e-9 by default: quadratic convergence
 // then leaves off-diagonal elements of order k * 1e-17 relative to the gaps) and
-// in which no rotated element was above 1e-8 of sqrt(|A_pp A_qq|).
+// in which no rotated element was above 1e-8 of sqrt(|A_pp A_qq|). If such a sweep
+// turned some pair by more than 2^-20 all the same (one that does not count: equal
+// diagonals, an element of rounding size), it takes a second such sweep, or one
+// that counts nothing: that rotation may bring back, at full size, an element that
+// a counted one has just taken away (clusters of equal eigenvalues: residuals of
+// 2e-12 with one such sweep, 1e-15 with two).
 #include <cooperative_groups.h>
 
 #include "../../include/itp2d_gpu.h"
@@ -68,6 +73,7 @@ struct Shared {
 	double2 re[2][NR];                           // e = c / |c|
 	int next[2];  // phase-2 item of each CTA half
 	int cnt;                                     // counted rotations of the current outer sweep
+	int mixed;                                   // a rotation by more than 2^-20 in it
 	unsigned long long tmax;                     // largest tangent (bits of a non-negative double)
 	// Subproblem buffer b, only the upper triangle (row <= column) in use.
 	__device__ double2* m(int b) { return op[3] + b * OP; }
@@ -120,6 +126,19 @@ __device__ __forceinline__ void half_rc(int lt, int b, int h, int& row, int& col
 // Barrier of one half of the CTA (named barrier 1 + half, 256 threads).
 __device__ __forceinline__ void half_sync(int half) {
 	asm volatile("bar.sync %0, %1;\n" ::"r"(1 + half), "r"(kThreads / 2) : "memory");
+}
+
+// Bit of a sweep's counter beside its counted rotations (fewer than 2^30).
+constexpr int kMixed = 1 << 30;
+
+// Whether a sweep with cnt counted rotations and largest tangent tm is the last;
+// small: whether the sweep before was below the tolerance too, replaced by this
+// one's. A tolerance looser than the default asks for no second sweep.
+__device__ __forceinline__ bool last_sweep(int cnt, bool mixed, double tm, double tau_final, bool& small) {
+	const bool below = tm < tau_final;
+	const bool last = cnt == 0 || (below && (!mixed || small || tau_final > kTauFinal));
+	small = below;
+	return last;
 }
 
 // Phase 1 for pair j of round t (within-sweep round rr): forms the subproblem
@@ -361,13 +380,13 @@ __global__ void __launch_bounds__(kThreads, 1) bjacobi_kernel(double2* A0, doubl
 	const bool join = split && nW > 8 * p2count;
 
 	if (tid == 0) {
-		sh.cnt = 0;
+		sh.cnt = sh.mixed = 0;
 		sh.tmax = 0ULL;
 	}
 	__syncthreads();
 
 	int sweep = 0;
-	bool stop = false, converged = false;
+	bool stop = false, converged = false, small = false;
 	// round t, t mod 3 and t mod rounds (64-bit remainders cost 1000 cycles a round)
 	long long t = 0;
 	int t3 = 0, rr = 0;
@@ -393,8 +412,9 @@ __global__ void __launch_bounds__(kThreads, 1) bjacobi_kernel(double2* A0, doubl
 		const bool sweep_end = do_p1 && rr == rounds - 1;
 		if (sweep_end && tid == 0) {
 			if (sh.cnt) atomicAdd(&counters[sweep], sh.cnt);
+			if (sh.mixed) atomicOr(&counters[sweep], kMixed);
 			if (sh.tmax) atomicMax(&tmax[sweep], sh.tmax);
-			sh.cnt = 0;
+			sh.cnt = sh.mixed = 0;
 			sh.tmax = 0ULL;
 		}
 		grid.sync();
@@ -403,7 +423,7 @@ __global__ void __launch_bounds__(kThreads, 1) bjacobi_kernel(double2* A0, doubl
 			// uniform across the grid: the counters are final after grid.sync
 			const int cnt = *((volatile int*)&counters[sweep]);
 			const double tm = __longlong_as_double((long long)*((volatile unsigned long long*)&tmax[sweep]));
-			if (cnt == 0 || tm < tau_final) {
+			if (last_sweep(cnt & (kMixed - 1), cnt >= kMixed, tm, tau_final, small)) {
 				converged = true;
 				stop = true;
 			}
@@ -441,9 +461,10 @@ __global__ void __launch_bounds__(32) tiny_jacobi_kernel(double2* A, double2* V,
 	}
 	__syncwarp();
 	int sweep = 0;
-	bool converged = false;
+	bool converged = false, small = false;
 	while (!converged && sweep < max_sweeps) {
 		int cnt = 0;
+		bool mixed = false;
 		double tmax = 0.0;
 #pragma unroll 1
 		for (int p = 0; p + 1 < n; p++)
@@ -452,6 +473,7 @@ __global__ void __launch_bounds__(32) tiny_jacobi_kernel(double2* A, double2* V,
 				double a = M[m_at(p, p)].x, b = M[m_at(q, q)].x;
 				double2 c = M[m_at(p, q)];
 				const Rotation<double> J = make_rotation<double>(a, b, c.x, c.y, tol, kNoiseRel, cnt, tmax);
+				mixed |= fabs(J.s) >= 0x1p-20;
 				rotated_pair(J, a, b, c.x, c.y);
 				__syncwarp();
 				if (i < n) {
@@ -474,7 +496,7 @@ __global__ void __launch_bounds__(32) tiny_jacobi_kernel(double2* A, double2* V,
 				__syncwarp();
 			}
 		sweep++;
-		converged = cnt == 0 || tmax < tau_final;  // the same in every lane
+		converged = last_sweep(cnt, mixed, tmax, tau_final, small);  // the same in every lane
 	}
 	for (int e = i; e < n * n; e += 32) {
 		const int r = e / n, l = e % n;

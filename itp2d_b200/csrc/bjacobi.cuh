@@ -292,7 +292,8 @@ __device__ __forceinline__ void cols2(R s, R tau, R er, R ei, R& xsr, R& xsi,
 // Offsets whose order is known in a cross sweep are formed without comparing
 // (with the round counters kept in 32 bits: 8 % of an eigensolve).
 // `sh`: m(b), the buffers of M; rst, re, the rotations; xch(), the exchange area
-// of the Q warps; cnt and tmax.
+// of the Q warps; cnt and tmax; in double precision mixed (one Q warp notes any
+// rotation by more than 2^-20).
 template <class R, bool FULL, bool QT, class SH>
 __device__ __forceinline__ void inner_sweep(SH& sh, R tol, R noise, c2<R>* Qg) {
 	using T = c2<R>;
@@ -467,6 +468,7 @@ __device__ __forceinline__ void inner_sweep(SH& sh, R tol, R noise, c2<R>* Qg) {
 			xp[h] = mk<R>(i0 + h == p0 ? 1.0 : 0.0, 0.0);
 			xq[h] = mk<R>(i0 + h == q0 ? 1.0 : 0.0, 0.0);
 		}
+		bool mixed = false;  // a rotation by more than 2^-20
 		// this warp's exchange area: [member][row h][half of the warp][column]
 		T* xch = sh.xch() + w * 4 * 2 * NR;
 		const int at = (lane >> 4) * NR, own = at + j, up = at + ((j + 1) & (NR - 1)), down = at + ((j - 1) & (NR - 1));
@@ -474,6 +476,7 @@ __device__ __forceinline__ void inner_sweep(SH& sh, R tol, R noise, c2<R>* Qg) {
 #pragma unroll 1
 		for (int r = 0; r < ROUNDS; r++) {
 			const T st = sh.rst[r & 1][j], e = sh.re[r & 1][j];
+			if constexpr (sizeof(R) == 8) mixed |= (__double2hiint(st.x) & 0x7FFFFFFF) >= (1023 - 20) << 20;
 #pragma unroll
 			for (int h = 0; h < 2; h++) cols2(st.x, st.y, e.x, e.y, xp[h].x, xp[h].y, xq[h].x, xq[h].y);
 			// the columns move on to the lanes of round r + 1's pairs
@@ -497,6 +500,9 @@ __device__ __forceinline__ void inner_sweep(SH& sh, R tol, R noise, c2<R>* Qg) {
 				}
 			}
 			__syncthreads();  // also: the exchange area is free again
+		}
+		if constexpr (sizeof(R) == 8) {
+			if (w == 0 && __any_sync(0xffffffffu, mixed) && lane == 0) sh.mixed = 1;
 		}
 		// after all rounds the columns are back at their places
 #pragma unroll
