@@ -110,6 +110,11 @@ cudaError_t launch_bjacobi32(const double2* S, int k, JacobiWork& w, int num_sms
 // consumed. Returns a CUDA error code of the launches (status goes to *st).
 cudaError_t launch_eigensolve(double2* S, int k, JacobiWork& w, double2* W, EigStatus* st, int num_sms,
 		cudaStream_t s);
+// Exponent e of the power of two by which the eigensolver entry points divide a
+// matrix of n x n complex values (column-major, upper triangle) whose largest
+// component is below 2^-400 or above 2^400, else 0: null eigenvalues and the sums
+// of products then stay clear of the subnormal numbers and of the overflow.
+int eigensolve_exponent(int n, const double* A);
 // Eigenvalues (ascending, w.evals), permutation (w.perm) and eigenvectors
 // (columns of w.V, kp x kp with kp = jacobi_kp(k)) without the
 // overlap checks unless check != 0; check 2 also accepts a solve that ended

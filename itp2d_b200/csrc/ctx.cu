@@ -1529,10 +1529,15 @@ int itp2d_hermitian_eigensolve(int n, const double* A, double* evals, double* ev
 	if (n < 1 || !A || !evals || !evecs) return ITP2D_E_INVALID;
 	CoopUser user;
 	const int kp = jacobi_kp(n);
+	const int exponent = eigensolve_exponent(n, A);
 	std::vector<double2> S((size_t)n * n);
 	for (int i = 0; i < n; i++)
 		for (int j = i; j < n; j++) {
-			const double re = A[2 * ((size_t)j * n + i)], im = A[2 * ((size_t)j * n + i) + 1];
+			double re = A[2 * ((size_t)j * n + i)], im = A[2 * ((size_t)j * n + i) + 1];
+			if (exponent) {
+				re = std::ldexp(re, -exponent);
+				im = std::ldexp(im, -exponent);
+			}
 			S[(size_t)i * n + j] = make_double2(re, i == j ? 0.0 : im);
 			S[(size_t)j * n + i] = make_double2(re, i == j ? 0.0 : -im);
 		}
@@ -1578,6 +1583,8 @@ int itp2d_hermitian_eigensolve(int n, const double* A, double* evals, double* ev
 		if (status == ITP2D_OK && hs.status != ITP2D_OK) status = hs.status;
 	}
 	if (status == ITP2D_OK) {
+		if (exponent)
+			for (int i = 0; i < n; i++) evals[i] = std::ldexp(evals[i], exponent);
 		const int jkp = jacobi_kp(n);
 		for (int m = 0; m < n; m++)
 			for (int i = 0; i < n; i++) {

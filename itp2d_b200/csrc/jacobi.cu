@@ -10,7 +10,9 @@
 // rounds of 16 x 16 rotations in shared memory, where one grid-wide round per
 // k/2 rotations (scalar cyclic Jacobi, 199 rounds of 8.8 us each) took 17.5 ms
 // per eigensolve.
+#include <algorithm>
 #include <atomic>
+#include <cmath>
 #include <mutex>
 
 #include "contract.cuh"
@@ -188,6 +190,16 @@ __global__ void ritz_w_kernel(const double2* __restrict__ V, int k, int kp, cons
 }
 
 }  // namespace
+
+int eigensolve_exponent(int n, const double* A) {
+	double top = 0.0;
+	for (int j = 0; j < n; j++)
+		for (int i = 0; i <= j; i++) {
+			const double* v = A + 2 * ((size_t)j * n + i);
+			top = std::max(top, std::max(std::fabs(v[0]), i == j ? 0.0 : std::fabs(v[1])));
+		}
+	return top > 0.0 && std::isfinite(top) && (top < 0x1p-400 || top > 0x1p400) ? std::ilogb(top) : 0;
+}
 
 size_t jacobi_counters(int max_sweeps) { return jacobi_counter_ints(max_sweeps); }
 

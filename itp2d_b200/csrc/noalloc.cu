@@ -19,6 +19,8 @@
 // device reset or a re-created primary context never leaves a stale address;
 // the first call on a device also loads this library's device code there, so
 // make that first call before any stream capture begins.
+#include <cmath>
+
 #include "../../include/itp2d_gpu.h"
 #include "contract.cuh"
 
@@ -66,13 +68,14 @@ int scratch_address(unsigned char** out) {
 }
 
 // Full Hermitian matrix (row-major) from the upper triangle of the
-// column-major input, the part ZHEEV("U") reads.
-__global__ void expand_upper_kernel(const double2* __restrict__ in, int n, double2* __restrict__ S) {
+// column-major input, the part ZHEEV("U") reads, divided by 2^exponent.
+__global__ void expand_upper_kernel(const double2* __restrict__ in, int n, int exponent, double2* __restrict__ S) {
 	const int idx = blockIdx.x * blockDim.x + threadIdx.x;
 	if (idx >= n * n) return;
 	const int i = idx / n, j = idx % n;
 	if (i > j) return;
-	const double2 v = in[(size_t)j * n + i];
+	double2 v = in[(size_t)j * n + i];
+	if (exponent) v = make_double2(scalbn(v.x, -exponent), scalbn(v.y, -exponent));
 	if (i == j) {
 		S[(size_t)i * n + i] = make_double2(v.x, 0.0);
 	} else {
@@ -122,7 +125,8 @@ extern "C" int itp2d_hermitian_eigensolve_noalloc(int n, const double* A, double
 	const int nn = n * n;
 	cudaError_t e = cudaMemcpy(in, A, (size_t)nn * sizeof(double2), cudaMemcpyHostToDevice);
 	if (e != cudaSuccess) return status_of(e);
-	expand_upper_kernel<<<(nn + 255) / 256, 256>>>(in, n, S);
+	const int exponent = itp2d::eigensolve_exponent(n, A);
+	expand_upper_kernel<<<(nn + 255) / 256, 256>>>(in, n, exponent, S);
 	e = itp2d::launch_eigh(S, n, w, dstat, sms, 0, 0);
 	if (e != cudaSuccess) return status_of(e);
 	gather_vectors_kernel<<<(nn + 255) / 256, 256>>>(w.V, n, kp, w.perm, vec);
@@ -132,5 +136,7 @@ extern "C" int itp2d_hermitian_eigensolve_noalloc(int n, const double* A, double
 	EigStatus hs;
 	if (e == cudaSuccess) e = cudaMemcpy(&hs, dstat, sizeof(EigStatus), cudaMemcpyDeviceToHost);
 	if (e != cudaSuccess) return status_of(e);
+	if (exponent)
+		for (int i = 0; i < n; i++) evals[i] = std::ldexp(evals[i], exponent);
 	return hs.status;
 }

@@ -65,3 +65,19 @@ def test_orthonormalisation_of_decayed_states(capi):
     out = c.download().reshape(k, -1)
     c.close()
     assert np.max(np.abs(out.conj() @ out.T * dx * dx - np.eye(k))) < 1e-13
+
+
+# null eigenvalues whose rounding would be subnormal, sums of products beside the
+# largest number
+@pytest.mark.parametrize("exponent", [-1000, -560, 560, 1015])
+@pytest.mark.parametrize("n,rank", [(5, 3), (20, 7), (40, 20), (130, 50), (260, 100)])
+def test_scaled_rank_deficient_matrices(capi, n, rank, exponent):
+    rng = np.random.default_rng([n, rank])
+    B = (rng.standard_normal((n, rank)) + 1j * rng.standard_normal((n, rank))) / np.sqrt(2 * n)
+    M = B @ B.conj().T
+    ev, U = capi.hermitian_eigensolve(np.ldexp(M.real, exponent) + 1j * np.ldexp(M.imag, exponent))
+    ev = np.ldexp(ev, -exponent)
+    top = np.max(np.abs(ev))
+    assert np.max(np.abs(ev - np.linalg.eigvalsh(M))) < 1e-13 * top
+    assert np.max(np.abs(U.conj().T @ U - np.eye(n))) < 2e-14
+    assert np.max(np.abs(M @ U - U * ev[None, :])) < 1e-13 * top
